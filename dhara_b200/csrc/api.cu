@@ -427,8 +427,33 @@ int encode_map(CUtensorMap *m, const void *array, size_t elt, const DomainDesc &
     return DHARA_OK;
 }
 
+// The pipelined solve's maps: STAGE_PLANES planes of `arrays` arrays, `apart`
+// elements from one to the next, in one box.
+int encode_pipe_map(CUtensorMap *m, const void *array, size_t elt, const DomainDesc &D, bool halo, int arrays = 1,
+                    long long apart = 0) {
+    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    if (!enc) return fail(DHARA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    const cuuint64_t dims[4] = {(cuuint64_t)D.nx, (cuuint64_t)D.ny, (cuuint64_t)D.nz, (cuuint64_t)arrays};
+    const cuuint64_t strides[3] = {(cuuint64_t)D.nxp * elt, (cuuint64_t)D.nxp * D.ny * elt, (cuuint64_t)apart * elt};
+    const int xoff = (int)(16 / elt);
+    const cuuint32_t box[4] = {(cuuint32_t)(halo ? D.tx + 2 * xoff : D.tx), (cuuint32_t)(halo ? D.ty + 2 : D.ty),
+                               STAGE_PLANES, (cuuint32_t)arrays};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    void *base = (void *)((const char *)array + (size_t)D.off3 * elt);
+    if (((uintptr_t)base & 15) != 0 || (strides[0] & 15) != 0 || (strides[2] & 15) != 0)
+        return fail(DHARA_ERR_INVALID, "internal: unaligned 3D array for TMA");
+    const CUtensorMapDataType dt = elt == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+    CUresult r = enc(m, dt, arrays > 1 ? 4 : 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(DHARA_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return DHARA_OK;
+}
+
 int build_tensor_maps(dhara_handle *h) {
     const DevPtrs &P = h->P;
+    const size_t sF = FACTOR_BYTES(h->mixed);
+    const long long N = h->Ntot;
     const size_t sT = h->mixed ? 4 : 8;
     const int chi = h->mixed ? CHUNK_F32 : CHUNK_F64;
     std::vector<CUtensorMap> maps((size_t)h->ndom * NMAP);
@@ -451,6 +476,20 @@ int build_tensor_maps(dhara_handle *h) {
         rc |= encode_map(m + MAP_K64_H, P.K64, 8, D, true, CH_R);
         rc |= encode_map(m + MAP_D64_O, P.D64, 8, D, false, CH_R);
         rc |= encode_map(m + MAP_B_O, P.b, 8, D, false, CH_R);
+        rc |= encode_pipe_map(m + PMAP_ZTP0_H, P.z0, sT, D, true, 3, N);
+        rc |= encode_pipe_map(m + PMAP_ZTP1_H, P.z1, sT, D, true, 3, N);
+        rc |= encode_pipe_map(m + PMAP_Z0_H, P.z0, sT, D, true);
+        rc |= encode_pipe_map(m + PMAP_Z1_H, P.z1, sT, D, true);
+        rc |= encode_pipe_map(m + PMAP_P0_H, P.p0, sT, D, true);
+        rc |= encode_pipe_map(m + PMAP_P1_H, P.p1, sT, D, true);
+        rc |= encode_pipe_map(m + PMAP_K_H, P.K, sT, D, true);
+        rc |= encode_pipe_map(m + PMAP_OWN_O, P.D, sT, D, false, sF == sT ? 4 : 2, N);
+        rc |= encode_pipe_map(m + PMAP_D_O, P.D, sT, D, false);
+        rc |= encode_pipe_map(m + PMAP_FAC_O, P.finv, sF, D, false, 2, N);
+        rc |= encode_pipe_map(m + PMAP_X64_H, P.x, 8, D, true);
+        rc |= encode_pipe_map(m + PMAP_K64_H, P.K64, 8, D, true);
+        rc |= encode_pipe_map(m + PMAP_D64_O, P.D64, 8, D, false);
+        rc |= encode_pipe_map(m + PMAP_B_O, P.b, 8, D, false);
         if (rc) return rc;
     }
     CUtensorMap *dm = const_cast<CUtensorMap *>(h->P.tmaps);
@@ -684,6 +723,7 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
         if (p.nz > h->nz_max) h->nz_max = p.nz;
         if (p.picard_maxiter > h->maxiter_picard) h->maxiter_picard = p.picard_maxiter;
     }
+    h->Ntot = (h->Ntot + 31) & ~31LL;  // arrays of one allocation start as aligned as its base
     // the inner sweeps index cells with 32-bit offsets
     if (h->Ntot >= (1LL << 31))
         return bail(fail(DHARA_ERR_UNSUPPORTED, "a handle holds at most 2^31 - 1 cells (with row padding); got %lld",
@@ -706,10 +746,26 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
     TileDesc *d_tiles = nullptr;
     rc |= dalloc(h, &d_tiles, h->tiles_cap);
     for (double **q : {&P.psin, &P.thetan, &P.psim, &P.x, &P.b, &P.ksat}) rc |= dalloc(h, q, N);
-    for (void **q : {&P.K, &P.D, &P.p0, &P.p1, &P.z0, &P.z1, &P.t0, &P.t1, &P.d})
-        rc |= dalloc_void(h, q, N * sT);
+    // sets of arrays that one TMA box copies are one allocation each: z, t, p
+    // (two of them), and the arrays read at a tile's own columns -- D, 1/den,
+    // c', d where the factors have the inner precision, else D, d and the factors
     const size_t sF = FACTOR_BYTES(h->mixed);
-    for (void **q : {&P.finv, &P.fc}) rc |= dalloc_void(h, q, N * sF);
+    char *ztp = nullptr, *own = nullptr, *fac = nullptr;
+    rc |= dalloc(h, &ztp, 6 * N * sT);
+    rc |= dalloc(h, &own, (sF == sT ? 4 : 2) * N * sT);
+    if (sF != sT) rc |= dalloc(h, &fac, 2 * N * sF);
+    rc |= dalloc_void(h, &P.K, N * sT);
+    if (rc) return bail(DHARA_ERR_NOMEM);
+    P.z0 = ztp;
+    P.t0 = ztp + N * sT;
+    P.p0 = ztp + 2 * N * sT;
+    P.z1 = ztp + 3 * N * sT;
+    P.t1 = ztp + 4 * N * sT;
+    P.p1 = ztp + 5 * N * sT;
+    P.D = own;
+    P.finv = fac ? fac : own + N * sT;
+    P.fc = fac ? fac + N * sF : own + 2 * N * sT;
+    P.d = own + (fac ? 1 : 3) * N * sT;
     if (h->mixed) {
         rc |= dalloc(h, &P.K64, N);
         rc |= dalloc(h, &P.D64, N);
@@ -868,7 +924,7 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
     h->L.nz_max = h->nz_max;
     h->L.mixed = h->mixed;
     h->L.olf_mg = params[0].overland_solver == 0 ? 1 : 0;
-    e = configure_3d(h->L, device, P.ntiles);
+    e = configure_3d(h->L, device, P.ntiles, P.ndom);
     if (e == cudaSuccess) e = configure_2d(h->L, device);
     if (e == cudaSuccess) e = configure_mg(h->L, device);
     if (e != cudaSuccess) return bail(fail(DHARA_ERR_CUDA, "kernel configuration: %s", cudaGetErrorString(e)));

@@ -112,105 +112,134 @@ __device__ __forceinline__ bool counter_sync(unsigned int *count, unsigned int t
     return counter_sync(count, target, gb, [] {});
 }
 
+// ------------------------------------------------------------ tile groups
+// Tiles are worked on by groups of TILE_THREADS threads: the whole block (G = 1)
+// in most kernels, G groups of a larger block in k_step_pipe.  These meet at a
+// named barrier each; one whose number is not known when the kernel is compiled
+// takes all 16 of the block's, of which an SM has 64 -- k_krylov's 7 blocks per SM
+// would be 4 (512x512x40 81.5 ms a pass instead of 52.6) -- so a block of one group
+// uses __syncthreads.
+template <int G>
+__device__ __forceinline__ int tile_thread() {
+    return G == 1 ? (int)threadIdx.x : (int)threadIdx.x & (TILE_THREADS - 1);
+}
+template <int G>
+__device__ __forceinline__ int tile_group() {
+    return G == 1 ? 0 : (int)threadIdx.x / TILE_THREADS;
+}
+template <int G>
+__device__ __forceinline__ void group_sync() {
+    if constexpr (G == 1) __syncthreads();
+    else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + tile_group<G>()), "n"(TILE_THREADS) : "memory");
+}
+
 // --------------------------------------------------------- reductions
-// Deterministic block sum of NV doubles (fixed warp/shuffle order); the
+// Deterministic group sum of NV doubles (fixed warp/shuffle order); the
 // result is returned in every thread.
-template <int NV>
+template <int NV, int G = 1>
 __device__ __forceinline__ void block_sum(double (&v)[NV]) {
-    __shared__ double s_w[NV][TILE_THREADS / 32];
-    __shared__ double s_out[NV];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ double s_w[G][NV][TILE_THREADS / 32];
+    __shared__ double s_out[G][NV];
+    const int lane = threadIdx.x & 31, warp = tile_thread<G>() >> 5, grp = tile_group<G>();
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         double a = v[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (lane == 0) s_w[i][warp] = a;
+        if (lane == 0) s_w[grp][i][warp] = a;
     }
-    __syncthreads();
-    if (threadIdx.x < NV) {
+    group_sync<G>();
+    if (tile_thread<G>() < NV) {
         double a = 0.0;
 #pragma unroll
-        for (int w = 0; w < TILE_THREADS / 32; ++w) a += s_w[threadIdx.x][w];
-        s_out[threadIdx.x] = a;
+        for (int w = 0; w < TILE_THREADS / 32; ++w) a += s_w[grp][tile_thread<G>()][w];
+        s_out[grp][tile_thread<G>()] = a;
     }
-    __syncthreads();
+    group_sync<G>();
 #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = s_out[i];
-    __syncthreads();
+    for (int i = 0; i < NV; ++i) v[i] = s_out[grp][i];
+    group_sync<G>();
 }
 
+template <int G>
 __device__ __forceinline__ double block_max(double v) {
-    __shared__ double s_w[TILE_THREADS / 32];
-    __shared__ double s_out;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ double s_w[G][TILE_THREADS / 32];
+    __shared__ double s_out[G];
+    const int lane = threadIdx.x & 31, warp = tile_thread<G>() >> 5, grp = tile_group<G>();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (lane == 0) s_w[warp] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = s_w[0];
-        for (int w = 1; w < TILE_THREADS / 32; ++w) a = fmax(a, s_w[w]);
-        s_out = a;
+    if (lane == 0) s_w[grp][warp] = v;
+    group_sync<G>();
+    if (tile_thread<G>() == 0) {
+        double a = s_w[grp][0];
+        for (int w = 1; w < TILE_THREADS / 32; ++w) a = fmax(a, s_w[grp][w]);
+        s_out[grp] = a;
     }
-    __syncthreads();
-    v = s_out;
-    __syncthreads();
+    group_sync<G>();
+    v = s_out[grp];
+    group_sync<G>();
     return v;
 }
 
-// Per-domain reduction across the tiles of a domain.  Every tile of the
-// domain calls it once (all threads, v already block-summed or not: it sums
-// the block itself).  The last tile to arrive sums the tiles' partials in
-// tile order -- the same order whichever tile is last, so the result is
-// bitwise reproducible -- and gets true with the domain totals in v.
-template <int NV, bool IS_MAX = false>
-__device__ __forceinline__ bool domain_reduce(const DevPtrs &P, int tile, int dom, int slot,
-                                              double (&v)[NV]) {
-    __shared__ int s_last;
+// Reduction across partials [begin, end) of a domain, kept in a list of
+// `stride`.  Each of them is contributed by one group (all its threads, v
+// already group-summed or not: it sums the group itself), at place `at`.  The
+// last group to arrive sums the partials in order -- the same order whichever
+// is last, so the result is bitwise reproducible -- and gets true with the
+// totals in v.
+template <int NV, bool IS_MAX = false, int G = 1>
+__device__ __forceinline__ bool tiles_reduce(const DevPtrs &P, int at, int begin, int end, int stride,
+                                             unsigned int *arrive, double (&v)[NV]) {
+    __shared__ int s_last[G];
     if (IS_MAX) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) v[i] = block_max(v[i]);
+        for (int i = 0; i < NV; ++i) v[i] = block_max<G>(v[i]);
     } else {
-        block_sum<NV>(v);
+        block_sum<NV, G>(v);
     }
-    if (threadIdx.x == 0) {
+    if (tile_thread<G>() == 0) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) __stcg(&P.partials[(size_t)i * P.ntiles + tile], v[i]);
+        for (int i = 0; i < NV; ++i) __stcg(&P.partials[(size_t)i * stride + at], v[i]);
         __threadfence();
-        const DomainDesc &D = P.dom[dom];
-        const unsigned int prev = atomicAdd(&P.arrive[dom * 4 + slot], 1u);
-        s_last = (prev == (unsigned int)(D.tile_end - D.tile_begin - 1));
+        const unsigned int prev = atomicAdd(arrive, 1u);
+        s_last[tile_group<G>()] = (prev == (unsigned int)(end - begin - 1));
     }
-    __syncthreads();
-    const bool last = s_last != 0;
-    __syncthreads();
+    group_sync<G>();
+    const bool last = s_last[tile_group<G>()] != 0;
+    group_sync<G>();
     if (!last) return false;
     __threadfence();
-    const DomainDesc &D = P.dom[dom];
     double acc[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) acc[i] = IS_MAX ? -INFINITY : 0.0;
-    // SoA partials: consecutive threads read consecutive tiles (coalesced) and
-    // the loop carries no dependence, so several loads are in flight.
+    // SoA partials: consecutive threads read consecutive partials (coalesced)
+    // and the loop carries no dependence, so several loads are in flight.
 #pragma unroll 4
-    for (int t = D.tile_begin + threadIdx.x; t < D.tile_end; t += blockDim.x) {
+    for (int t = begin + tile_thread<G>(); t < end; t += TILE_THREADS) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const double w = __ldcg(&P.partials[(size_t)i * P.ntiles + t]);
+            const double w = __ldcg(&P.partials[(size_t)i * stride + t]);
             acc[i] = IS_MAX ? fmax(acc[i], w) : acc[i] + w;
         }
     }
     if (IS_MAX) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) acc[i] = block_max(acc[i]);
+        for (int i = 0; i < NV; ++i) acc[i] = block_max<G>(acc[i]);
     } else {
-        block_sum<NV>(acc);
+        block_sum<NV, G>(acc);
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = acc[i];
-    if (threadIdx.x == 0) P.arrive[dom * 4 + slot] = 0u;
+    if (tile_thread<G>() == 0) *arrive = 0u;
     return true;
+}
+
+// The same with one partial per tile.
+template <int NV, bool IS_MAX = false, int G = 1>
+__device__ __forceinline__ bool domain_reduce(const DevPtrs &P, int tile, int dom, int slot,
+                                              double (&v)[NV]) {
+    const DomainDesc &D = P.dom[dom];
+    return tiles_reduce<NV, IS_MAX, G>(P, tile, D.tile_begin, D.tile_end, P.ntiles, &P.arrive[dom * 4 + slot], v);
 }
 
 // ---------------------------------------------------- branch signature
@@ -394,6 +423,7 @@ struct ColumnRef {
     bool valid;
 };
 
+template <int G = 1>
 __device__ __forceinline__ ColumnRef column_of(const DevPtrs &P, int tile) {
     const TileDesc t = P.tiles[tile];
     const DomainDesc &D = P.dom[t.dom];
@@ -402,8 +432,8 @@ __device__ __forceinline__ ColumnRef column_of(const DevPtrs &P, int tile) {
     r.tx = D.tx;
     r.ty = D.ty;
     r.tx_log2 = D.tx_log2;
-    r.i = t.x0 + ((int)threadIdx.x & (D.tx - 1));
-    r.j = t.y0 + ((int)threadIdx.x >> D.tx_log2);
+    r.i = t.x0 + (tile_thread<G>() & (D.tx - 1));
+    r.j = t.y0 + (tile_thread<G>() >> D.tx_log2);
     r.nx = D.nx;
     r.ny = D.ny;
     r.nz = D.nz;

@@ -67,6 +67,13 @@
 #define KRYLOV_DSMEM_F32 0
 #endif
 
+// Pipelined solve (pipe_solve.cuh): threads of a block -- 4 column warps, 8 plane
+// warps, two producer warps and the observer warp -- planes of a ring stage, most
+// stages of a ring
+#define SOLVE_THREADS (TILE_THREADS + 256 + 96)
+#define STAGE_PLANES 2
+#define RING_MAX 32
+
 // Tensor maps of one domain (index = dom * NMAP + id): halo boxes
 // (TILE_X + 32 bytes) x (TILE_Y + 2) x chunk, own boxes TILE_X x TILE_Y x chunk.
 // The inner iteration's vectors z, t = M^-1 A p and p are double buffered
@@ -76,7 +83,21 @@ enum {
     MAP_P0_H = 0, MAP_P1_H, MAP_Z0_H, MAP_Z1_H, MAP_T0_H, MAP_T1_H, MAP_K_H,  // inner precision, halo
     MAP_D_O, MAP_DD_O, MAP_INV_O, MAP_C_O,                                    // inner precision, own
     MAP_X64_H, MAP_K64_H, MAP_D64_O, MAP_B_O,                                 // FP64 outer residual
+    // the pipelined solve's, STAGE_PLANES high; z, t, p of a set and the own arrays
+    // are one allocation each, so that one box copies all of a set
+    PMAP_ZTP0_H, PMAP_ZTP1_H,                    // z, t, p of a set (halo)
+    PMAP_Z0_H, PMAP_Z1_H, PMAP_P0_H, PMAP_P1_H,  // z or p alone
+    PMAP_K_H,
+    PMAP_OWN_O,                                  // mixed: D, 1/den, c', d; FP64 mode: D, d
+    PMAP_D_O, PMAP_FAC_O,                        // D; 1/den and c'
+    PMAP_X64_H, PMAP_K64_H, PMAP_D64_O, PMAP_B_O,
     NMAP
+};
+
+// A solver pipeline's shared memory: column buffers (nb of colb bytes), then
+// the ring (n stages of `stage` bytes).
+struct PipeShape {
+    int n, stage, nb, colb;
 };
 
 // Per-domain constants (device copy in DevPtrs::dom).  3D arrays are stored
@@ -230,7 +251,7 @@ struct GlobalCtrl {
     unsigned int olf_bar;  // arrivals at the resident overland solve's barrier
     int olf_live[4];     // domains still iterating, rotating over three phases
     int n_picard;        // domains whose Picard iteration is not done this step (k_step)
-    int pad_g;
+    unsigned int kry_bar;  // arrivals at the pipelined solve's barrier (zeroed by the assembly before it)
 };
 
 // Number of double partial sums per tile kept for reductions.
@@ -244,6 +265,7 @@ struct DevPtrs {
     int ntiles, ndom;
     int smem_nz;         // column capacity of the d' buffer of the column solves in shared memory
     int pad_smem;
+    PipeShape pipe_c, pipe_r;  // the pipelined solve's inner sweeps and phase R (set at launch)
     // 3D double state
     double *psin, *thetan, *psim, *x, *b, *ksat, *alpha, *nvg;
     // FP64 coefficients of the outer residual (alias K, D in FP64 mode)
@@ -312,6 +334,8 @@ struct LaunchCfg {
     int olf_stream_per_sm_max, olf_stream_per_sm;
     int olf_allow_resident;
     int smem_3d;          // dynamic shared memory bytes of the 3D solve
+    int smem_pipe;        // dynamic shared memory a block of the pipelined solve may take
+    int pipe;             // 1: the solves run as the pipeline (pipe_solve.cuh)
     int nz_max;
     int mixed;
     int step_per_sm;      // co-resident blocks per SM of the fused step kernel
@@ -401,5 +425,5 @@ cudaError_t launch_adj_initial(const DevPtrs &P, const AdjPtrs &A, cudaStream_t 
 cudaError_t launch_layer_stats(const DevPtrs &P, double *part, int nz_max, double *hist, int max_steps,
                                cudaStream_t s);
 
-cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles);
+cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom);
 cudaError_t configure_2d(LaunchCfg &L, int device);

@@ -56,6 +56,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
                  : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {
     unsigned done;
     asm volatile(
@@ -83,6 +87,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, GridBa
     }
 }
 
+// The same for a warp that may wait long beside busy ones: the thread sleeps until
+// the phase completes or the hinted time is over, instead of polling.
+#define MBAR_HINT_NS 100000u
+__device__ __forceinline__ bool mbar_sleep(uint64_t *bar, unsigned parity, GridBarrier *gb) {
+    auto ready = [&]() {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred P;\n mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\n selp.u32 %0, 1, 0, P;\n}\n"
+            : "=r"(done)
+            : "r"(smem_addr(bar)), "r"(parity), "r"(MBAR_HINT_NS)
+            : "memory");
+        return done != 0;
+    };
+    if (ready()) return true;
+    if (*(volatile int *)&gb->error) return false;
+    const unsigned long long t0 = global_ns();
+    for (unsigned spins = 1;; ++spins) {
+        if (ready()) return true;
+        if ((spins & 15u) == 0 && global_ns() - t0 > MBAR_TIMEOUT_NS) {
+            atomicExch(&gb->error, 1);
+            return false;
+        }
+    }
+}
+
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z,
                                             uint64_t *bar) {
     asm volatile(
@@ -90,6 +119,20 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
         "[%5];\n" ::"r"(smem_addr(dst)),
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
         : "memory");
+}
+
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int x, int y, int z,
+                                            uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];\n" ::"r"(smem_addr(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(0), "r"(smem_addr(bar))
+        : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap *map, int x, int y, int z) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(map), "r"(x),
+                 "r"(y), "r"(z), "r"(0)
+                 : "memory");
 }
 
 // L2 prefetch of the box a load at the same coordinates would copy: no shared

@@ -22,7 +22,46 @@
 
 #include <cstdio>
 
-#define MAX_CYCLES 30
+// Storage type of the column preconditioner's factors 1/den and c': bf16 in
+// mixed mode with FACTOR_NARROW_F32, FP32 in FP64 mode with FACTOR_NARROW_F64.  Any rounding of
+// the stored pair still defines a symmetric positive definite M = L D L^T
+// (D = 1/inv > 0, L from c'), and every use of M -- phase R's z = M^-1 r,
+// the sweep's forward and back substitutions and its z.M z -- goes through
+// the stored values, so the inner CG sees one fixed preconditioner.
+template <typename T>
+struct Fac {
+    using type = T;
+};
+#if FACTOR_NARROW_F32
+template <>
+struct Fac<float> {
+    using type = __nv_bfloat16;
+};
+#endif
+#if FACTOR_NARROW_F64
+template <>
+struct Fac<double> {
+    using type = float;
+};
+#endif
+
+template <typename T>
+__device__ __forceinline__ T recip(T x);
+template <>
+__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
+template <>
+__device__ __forceinline__ double recip(double x) { return 1.0 / x; }
+
+// a / b where the quotient only feeds a sum of positive terms (z.M z): the
+// hardware reciprocal's approximation (about 2 ulp) in FP32
+template <typename T>
+__device__ __forceinline__ T quot(T a, T b);
+template <>
+__device__ __forceinline__ float quot(float a, float b) { return __fdividef(a, b); }
+template <>
+__device__ __forceinline__ double quot(double a, double b) { return a / b; }
+
+#include "pipe_solve.cuh"
 
 // The closure of the assembled system: the reference's FP64 expressions in
 // FP64 mode, the reformulated FP64 closure in mixed mode, or the FP32 closure
@@ -87,11 +126,12 @@ __global__ void k_prepare(DevPtrs P) {
 // IdentifyTopBoundary (206-257).  The top flux does not change between Picard
 // iterations (its inputs hpoten, qcapa, theta^n, Ks are fixed for the step), so
 // it is evaluated once per step.  Also resets the per-step control state.
+template <int G = 1>
 __device__ __forceinline__ void prologue_tile(const DevPtrs &P, int tile) {
-    const ColumnRef cr = column_of(P, tile);
+    const ColumnRef cr = column_of<G>(P, tile);
     const DomainDesc &D = P.dom[cr.dom];
     const TileDesc td = P.tiles[tile];
-    if (threadIdx.x == 0) {
+    if (tile_thread<G>() == 0) {
         if (tile == 0) {
             P.gctrl->n_active = 0;
             P.gctrl->n_inner_active = 0;
@@ -163,14 +203,15 @@ __global__ void k_prologue(DevPtrs P) {
 // (q_b = K of the bottom cell, written to bcqb as the reference does).
 // Eight blocks per SM (64 registers): the FP64 closure's latency chains need the
 // warps more than the registers (measured 18 % faster than the uncapped 96).
-template <typename T>
+template <typename T, int G = 1>
 __device__ __forceinline__ void assemble_tile(const DevPtrs &P, int tile) {
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
     const PicardCtrl &pc = P.pctrl[td.dom];
     const int done = pc.done;
     const int iter = pc.iter;
-    if (threadIdx.x == 0 && tile == D.tile_begin) {
+    if (tile_thread<G>() == 0 && tile == 0) P.gctrl->kry_bar = 0;
+    if (tile_thread<G>() == 0 && tile == D.tile_begin) {
         KrylovCtrl &kc = P.kctrl[td.dom];
         kc.active = done ? 0 : 1;
         kc.inner_active = 0;
@@ -183,7 +224,7 @@ __device__ __forceinline__ void assemble_tile(const DevPtrs &P, int tile) {
         if (!done) atomicAdd(&P.gctrl->n_active, 1);
     }
     if (done) return;
-    const ColumnRef cr = column_of(P, tile);
+    const ColumnRef cr = column_of<G>(P, tile);
     if (records(D, BR_SATURATION)) {
         // saturation (psi >= 0 switches the closure's branch) of every cell at psi^m
         unsigned long long bsig = 0;
@@ -355,12 +396,12 @@ __device__ __forceinline__ bool dir_rules(const ColumnRef &cr, int k, const DirF
 }
 
 // Pass 1: identity rows (D = -1, x = b = the row's right-hand side).
-template <typename T>
+template <typename T, int G = 1>
 __device__ __forceinline__ void dir_fixed_tile(const DevPtrs &P, int tile) {
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
     if (!D.has_dirichlet || P.pctrl[td.dom].done) return;
-    const ColumnRef cr = column_of(P, tile);
+    const ColumnRef cr = column_of<G>(P, tile);
     if (!cr.valid) return;
     long long g = cr.g0;
     for (int k = 0; k < cr.nz; ++k, g += cr.sxy) {
@@ -382,12 +423,12 @@ __global__ void __launch_bounds__(TILE_THREADS) k_dir_fixed(DevPtrs P) {
 
 // Pass 2: the rows next to identity rows get the reference's elimination
 // terms, less the coupling the matrix-free stencil applies to the fixed value.
-template <typename T>
+template <typename T, int G = 1>
 __device__ __forceinline__ void dir_rows_tile(const DevPtrs &P, int tile) {
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
     if (!D.has_dirichlet || P.pctrl[td.dom].done) return;
-    const ColumnRef cr = column_of(P, tile);
+    const ColumnRef cr = column_of<G>(P, tile);
     if (!cr.valid) return;
     const double ix2 = 1.0 / (D.dx * D.dx), iy2 = 1.0 / (D.dy * D.dy), iz2 = 1.0 / (D.dz * D.dz);
     long long g = cr.g0;
@@ -461,28 +502,6 @@ struct Chunk {
     static constexpr int inner = sizeof(T) == 4 ? CHUNK_F32 : CHUNK_F64;
 };
 
-// Storage type of the column preconditioner's factors 1/den and c': bf16 in
-// mixed mode with FACTOR_NARROW_F32, FP32 in FP64 mode with FACTOR_NARROW_F64.  Any rounding of
-// the stored pair still defines a symmetric positive definite M = L D L^T
-// (D = 1/inv > 0, L from c'), and every use of M -- phase R's z = M^-1 r,
-// the sweep's forward and back substitutions and its z.M z -- goes through
-// the stored values, so the inner CG sees one fixed preconditioner.
-template <typename T>
-struct Fac {
-    using type = T;
-};
-#if FACTOR_NARROW_F32
-template <>
-struct Fac<float> {
-    using type = __nv_bfloat16;
-};
-#endif
-#if FACTOR_NARROW_F64
-template <>
-struct Fac<double> {
-    using type = float;
-};
-#endif
 template <typename T, typename F>
 __device__ __forceinline__ T fac_get(F v) {
     if constexpr (std::is_same<F, __nv_bfloat16>::value) return (T)__bfloat162float(v);
@@ -608,22 +627,6 @@ __device__ __forceinline__ void back_sweep(const ColumnRef &cr, const T *s_d, co
         }
     }
 }
-
-template <typename T>
-__device__ __forceinline__ T recip(T x);
-template <>
-__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
-template <>
-__device__ __forceinline__ double recip(double x) { return 1.0 / x; }
-
-// a / b where the quotient only feeds a sum of positive terms (z.M z): the
-// hardware reciprocal's approximation (about 2 ulp) in FP32
-template <typename T>
-__device__ __forceinline__ T quot(T a, T b);
-template <>
-__device__ __forceinline__ float quot(float a, float b) { return __fdividef(a, b); }
-template <>
-__device__ __forceinline__ double quot(double a, double b) { return a / b; }
 
 // Face masks of a column: 1 where the face is interior, 0 on a domain face.
 struct Masks {
@@ -1200,16 +1203,17 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? KRYLOV_BLOCKS_F
 // ---------------------------------------------------------- Picard check
 // Max of |(psi^{m+1}-psi^m)/psi^{m+1}| (or the theta / absolute variants) per
 // domain, then the convergence decision and iteration bookkeeping.
+template <int G = 1>
 __device__ __forceinline__ void picard_check_tile(const DevPtrs &P, int tile) {
     const TileDesc td = P.tiles[tile];
-    if (tile == 0 && threadIdx.x == 0) {
+    if (tile == 0 && tile_thread<G>() == 0) {
         P.gctrl->n_active = 0;
         P.gctrl->n_inner_active = 0;
     }
     const PicardCtrl &pc = P.pctrl[td.dom];
     if (pc.done) return;
     const DomainDesc &D = P.dom[td.dom];
-    const ColumnRef cr = column_of(P, tile);
+    const ColumnRef cr = column_of<G>(P, tile);
     double mx = 0.0;
     int nonfinite = 0;
     if (cr.valid) {
@@ -1234,7 +1238,7 @@ __device__ __forceinline__ void picard_check_tile(const DevPtrs &P, int tile) {
     }
     if (nonfinite) atomicOr(&P.diag[td.dom].nonfinite, 1);
     double v[1] = {mx};
-    if (domain_reduce<1, true>(P, tile, td.dom, 1, v) && threadIdx.x == 0) {
+    if (domain_reduce<1, true, G>(P, tile, td.dom, 1, v) && tile_thread<G>() == 0) {
         PicardCtrl &c = P.pctrl[td.dom];
         DevDiag &dg = P.diag[td.dom];
         const KrylovCtrl &kc = P.kctrl[td.dom];
@@ -1263,11 +1267,11 @@ __global__ void __launch_bounds__(TILE_THREADS) k_picard_check(DevPtrs P) {
 // 809-826) and the rollover (833-840).  Interior face fluxes of the
 // reference's balance cancel pairwise (q_e of cell i equals q_w of cell i+1
 // bit for bit), so only boundary faces are summed.
-template <typename T>
+template <typename T, int G = 1>
 __device__ __forceinline__ void epilogue_tile(const DevPtrs &P, int tile) {
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
-    const ColumnRef cr = column_of(P, tile);
+    const ColumnRef cr = column_of<G>(P, tile);
     // v: 0 sum dtheta*dz, 1 dt*sum ssflux, 2 sum transp, 3 dt*boundary flux,
     //    4 storage (telescoping), 5 dt*q_top, 6 dt*q_bottom, 7 rain, 8 nonfinite
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -1329,7 +1333,7 @@ __device__ __forceinline__ void epilogue_tile(const DevPtrs &P, int tile) {
                                band3(P.hpoten[cr.c], qt * dt, rel_band(P.hpoten[cr.c], qt * dt, 1e-15)));
     }
     if (D.record_branches) branch_commit(&P.diag[td.dom].branch_sig, bsig);
-    if (domain_reduce<9>(P, tile, td.dom, 2, v) && threadIdx.x == 0) {
+    if (domain_reduce<9, false, G>(P, tile, td.dom, 2, v) && tile_thread<G>() == 0) {
         DevDiag &dg = P.diag[td.dom];
         PicardCtrl &pc = P.pctrl[td.dom];
         const double mb = v[0] + v[3] - v[2] + v[1];
@@ -1367,16 +1371,40 @@ __global__ void __launch_bounds__(TILE_THREADS) k_epilogue(DevPtrs P) {
 // keeps the registers it has in k_krylov.
 enum StepPhase { PH_PROLOGUE, PH_ASSEMBLE, PH_DIR_FIXED, PH_DIR_ROWS, PH_CHECK, PH_EPILOGUE };
 
-template <typename T, int PH>
+// GROUPS: tiles a block works on at the same time.
+template <typename T, int PH, int GROUPS>
 __device__ __noinline__ void step_phase(const DevPtrs &P) {
-    for (int t = blockIdx.x; t < P.ntiles; t += gridDim.x) {
-        if constexpr (PH == PH_PROLOGUE) prologue_tile(P, t);
-        else if constexpr (PH == PH_ASSEMBLE) assemble_tile<T>(P, t);
-        else if constexpr (PH == PH_DIR_FIXED) dir_fixed_tile<T>(P, t);
-        else if constexpr (PH == PH_DIR_ROWS) dir_rows_tile<T>(P, t);
-        else if constexpr (PH == PH_CHECK) picard_check_tile(P, t);
-        else epilogue_tile<T>(P, t);
+    if (tile_group<GROUPS>() >= GROUPS) return;
+    for (int t = blockIdx.x * GROUPS + tile_group<GROUPS>(); t < P.ntiles; t += gridDim.x * GROUPS) {
+        if constexpr (PH == PH_PROLOGUE) prologue_tile<GROUPS>(P, t);
+        else if constexpr (PH == PH_ASSEMBLE) assemble_tile<T, GROUPS>(P, t);
+        else if constexpr (PH == PH_DIR_FIXED) dir_fixed_tile<T, GROUPS>(P, t);
+        else if constexpr (PH == PH_DIR_ROWS) dir_rows_tile<T, GROUPS>(P, t);
+        else if constexpr (PH == PH_CHECK) picard_check_tile<GROUPS>(P, t);
+        else epilogue_tile<T, GROUPS>(P, t);
     }
+}
+
+// solve(): the linear solve of one Picard iteration.
+template <typename T, int GROUPS, typename Solve>
+__device__ __forceinline__ void run_step(const DevPtrs &P, int maxiter, int dirichlet, Solve solve) {
+    step_phase<T, PH_PROLOGUE, GROUPS>(P);
+    if (!grid_sync(P.barrier)) return;
+    for (int m = 0; m < maxiter; ++m) {
+        step_phase<T, PH_ASSEMBLE, GROUPS>(P);
+        if (!grid_sync(P.barrier)) return;
+        if (dirichlet) {
+            step_phase<T, PH_DIR_FIXED, GROUPS>(P);
+            if (!grid_sync(P.barrier)) return;
+            step_phase<T, PH_DIR_ROWS, GROUPS>(P);
+            if (!grid_sync(P.barrier)) return;
+        }
+        if (!solve()) return;
+        step_phase<T, PH_CHECK, GROUPS>(P);
+        if (!grid_sync(P.barrier)) return;
+        if (ldcg(&P.gctrl->n_picard) == 0) break;
+    }
+    step_phase<T, PH_EPILOGUE, GROUPS>(P);
 }
 
 template <typename T, int TXC>
@@ -1387,23 +1415,24 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? KRYLOV_BLOCKS_F
     constexpr bool DSMEM = sizeof(T) == 4 && KRYLOV_DSMEM_F32;
     const SolveSmem<T> sm = solve_smem<T, DSMEM>(P, smem_raw, s_bar);
     StageBars sb{s_bar, 0u, P.barrier, 0u};
-    step_phase<T, PH_PROLOGUE>(P);
-    if (!grid_sync(P.barrier)) return;
-    for (int m = 0; m < maxiter; ++m) {
-        step_phase<T, PH_ASSEMBLE>(P);
-        if (!grid_sync(P.barrier)) return;
-        if (dirichlet) {
-            step_phase<T, PH_DIR_FIXED>(P);
-            if (!grid_sync(P.barrier)) return;
-            step_phase<T, PH_DIR_ROWS>(P);
-            if (!grid_sync(P.barrier)) return;
-        }
-        if (!krylov_solve<T, DSMEM, TXC>(P, sm, sb)) return;
-        step_phase<T, PH_CHECK>(P);
-        if (!grid_sync(P.barrier)) return;
-        if (ldcg(&P.gctrl->n_picard) == 0) break;
-    }
-    step_phase<T, PH_EPILOGUE>(P);
+    run_step<T, 1>(P, maxiter, dirichlet, [&]() { return krylov_solve<T, DSMEM, TXC>(P, sm, sb); });
+}
+
+// The same kernels with the pipelined solve.
+template <typename T, int TXC>
+__global__ void __launch_bounds__(SOLVE_THREADS, 1) k_krylov_pipe(const __grid_constant__ DevPtrs P) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(8) pipe::PipeShared sh;
+    pipe::SolveBlock b = pipe::solve_block(P, smem_raw, &sh);
+    pipe::solve<T, TXC>(P, b);
+}
+template <typename T, int TXC>
+__global__ void __launch_bounds__(SOLVE_THREADS, 1)
+    k_step_pipe(const __grid_constant__ DevPtrs P, int maxiter, int dirichlet) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(8) pipe::PipeShared sh;
+    pipe::SolveBlock b = pipe::solve_block(P, smem_raw, &sh);
+    run_step<T, STEP_GROUPS>(P, maxiter, dirichlet, [&]() { return pipe::solve<T, TXC>(P, b); });
 }
 
 // Evaluates the closure at psi^n into out: which = 0 theta, 1 K, 2 C.
@@ -1537,7 +1566,86 @@ const void *step_kernel(const LaunchCfg &L, int uniform_tx) {
                                                                               : step_fn<0>(L.mixed);
 }
 
+template <int TXC>
+const void *pipe_fn(int mixed, bool step) {
+    return step ? (mixed ? (const void *)k_step_pipe<float, TXC> : (const void *)k_step_pipe<double, TXC>)
+                : (mixed ? (const void *)k_krylov_pipe<float, TXC> : (const void *)k_krylov_pipe<double, TXC>);
+}
+const void *pipe_kernel(const LaunchCfg &L, bool step) {
+    return L.uniform_tx == TILE_X ? pipe_fn<TILE_X>(L.mixed, step)
+           : L.uniform_tx == 16   ? pipe_fn<16>(L.mixed, step)
+                                  : pipe_fn<0>(L.mixed, step);
+}
+
+// Pipelines and grid of a solve: one block per SM, or per tile where there are
+// fewer.  Two column buffers when blocks have more than one tile and a ring of
+// PIPE_RING_LEAST stages still fits beside them (fewer keep too few bytes in
+// flight); the ring takes the rest, up to a whole column where a block has one
+// tile.  False where no such ring fits (columns of over 48 layers in FP64 mode).
+#define PIPE_RING_LEAST 6
+// shared memory the kernels declare: PipeShared and the step phases' reductions
+#define PIPE_STATIC_SMEM ((int)sizeof(pipe::PipeShared) + 2048)
+template <typename T>
+bool pipe_shapes(const LaunchCfg &L, int ntiles, PipeShape &c, PipeShape &r, int &smem) {
+    const int room = L.smem_pipe - 128;  // alignment
+    c.stage = (int)pipe::Stage<T>::bytes;
+    r.stage = (int)pipe::StageR<T>::bytes;
+    c.colb = r.colb = pipe::col_bytes(L.nz_max, sizeof(T));
+    const int whole = pipe::units_of(L.nz_max) < 3 ? 3 : pipe::units_of(L.nz_max);
+    const int most = ntiles > L.sms ? RING_MAX : whole;
+    bool fits = true;
+    smem = 0;
+    for (PipeShape *q : {&c, &r}) {
+        q->nb = ntiles > L.sms && (room - 2 * q->colb) / q->stage >= PIPE_RING_LEAST ? 2 : 1;
+        q->n = (room - q->nb * q->colb) / q->stage;
+        if (q->n > most) q->n = most;
+        fits = fits && q->n >= (most < PIPE_RING_LEAST ? most : PIPE_RING_LEAST);
+        const int use = q->nb * q->colb + q->n * q->stage;
+        smem = use > smem ? use : smem;
+    }
+    smem += 128;
+    return fits;
+}
+bool pipe_shapes(const LaunchCfg &L, int ntiles, PipeShape &c, PipeShape &r, int &smem) {
+    return L.mixed ? pipe_shapes<float>(L, ntiles, c, r, smem) : pipe_shapes<double>(L, ntiles, c, r, smem);
+}
+
+// Whether a handle's solves run as the pipeline (pipe_solve.cuh).  Its time goes
+// with the tiles of the SM that has most of them, krylov_solve's with the rounds
+// its blocks make: measured, a round takes as long as 6.4 tiles of the pipeline
+// (mixed), 3.7 (FP64 mode; 3.3 where a block's tiles are of several domains, whose
+// sums are formed one after the other).  Solves of a pass, krylov_solve / pipeline
+// in ms, tiles per SM (t) against rounds (r): mixed 301x211x33 14.9 / 12.5 (t 5, r
+// 1), 384x384x40 48.0 / 32.9 (8, 2), 448x448x40 50.0 / 45.0 (11, 2), 512x512x40 50.9
+// / 53.5 (14, 2), 576x576x40 80.3 / 78.2 (18, 3), 700x700x40 103 / 113 (27, 4); 64
+// domains 59.8 / 53.6 (19, 3), 80 71.6 / 73.8 (26, 4); FP64 272x272x40 21.9 / 22.9
+// (4, 1), 400x400x40 59.4 / 48.6 (9, 3), 512x512x40 76.0 / 71.2 (14, 4), 640x640x40
+// 127 / 122 (22, 6), 768x768x40 169 / 169 (32, 8); 48 domains 18.3 / 17.2 (6, 2), 64
+// 18.3 / 19.7 (7, 2).  Above 26 tiles per SM the two are within 5 % or krylov_solve
+// is ahead (256 domains 192 / 210).
+bool use_pipe(const LaunchCfg &L, int ntiles, int ndom) {
+    PipeShape c, r;
+    int smem;
+    const int tiles = (ntiles + L.sms - 1) / L.sms;
+    const int rounds = (ntiles + L.coop_blocks_3d - 1) / L.coop_blocks_3d;
+    const double round = L.mixed ? 6.4 : ndom > 1 ? 3.3 : 3.7;
+    return tiles <= 26 && tiles <= round * rounds && pipe_shapes(L, ntiles, c, r, smem);
+}
+
+cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int maxiter, int dirichlet, bool step, cudaStream_t s) {
+    DevPtrs args = P;
+    int smem = 0;
+    const int grid = L.sms < P.ntiles ? L.sms : P.ntiles;
+    if (!pipe_shapes(L, P.ntiles, args.pipe_c, args.pipe_r, smem)) return cudaErrorInvalidConfiguration;
+    const void *fn = pipe_kernel(L, step);
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem_pipe);
+    if (e != cudaSuccess) return e;
+    void *kargs[] = {&args, &maxiter, &dirichlet};
+    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SOLVE_THREADS), kargs, (size_t)smem, s);
+}
+
 cudaError_t launch_krylov(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s) {
+    if (L.pipe) return launch_pipe(P, L, 0, 0, false, s);
     DevPtrs args = P;
     void *kargs[] = {&args};
     const int blocks = L.krylov_per_sm * L.sms;
@@ -1547,6 +1655,7 @@ cudaError_t launch_krylov(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s) 
 }
 
 cudaError_t launch_step(const DevPtrs &P, const LaunchCfg &L, int maxiter, int dirichlet, cudaStream_t s) {
+    if (L.pipe) return launch_pipe(P, L, maxiter, dirichlet, true, s);
     DevPtrs args = P;
     void *kargs[] = {&args, &maxiter, &dirichlet};
     const int blocks = (L.krylov_per_sm < L.step_per_sm ? L.krylov_per_sm : L.step_per_sm) * L.sms;
@@ -1555,7 +1664,7 @@ cudaError_t launch_step(const DevPtrs &P, const LaunchCfg &L, int maxiter, int d
                                        (size_t)L.smem_3d, s);
 }
 
-cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles) {
+cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom) {
     cudaDeviceProp prop;
     cudaError_t e = cudaGetDeviceProperties(&prop, device);
     if (e != cudaSuccess) return e;
@@ -1579,6 +1688,9 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles) {
         }
     }
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    // the pipeline's kernels are not set up here: each is loaded when it is first
+    // launched (all six cost 19 ms of a process's first handle)
+    L.smem_pipe = (int)prop.sharedMemPerBlockOptin - PIPE_STATIC_SMEM;
     L.coop_blocks_3d = per_sm * prop.multiProcessorCount;
     L.sms = prop.multiProcessorCount;
     L.krylov_per_sm_max = per_sm;
@@ -1586,8 +1698,10 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles) {
     L.step_per_sm = step_sm < per_sm ? step_sm : per_sm;
     if (L.step_per_sm < 1) return cudaErrorInvalidConfiguration;
     // one launch per subsurface step by default, where the fused kernel keeps
-    // the Krylov kernel's occupancy
-    L.fused_step = L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
-    (void)ntiles;
+    // the Krylov kernel's occupancy; the pipelined solve's block has too few warps
+    // for the assembly (32x32x20 FP64 two steps 6.1 fused, 5.75 ms separate,
+    // 512x512x40 FP64 92 / 84.7)
+    L.pipe = use_pipe(L, ntiles, ndom);
+    L.fused_step = !L.pipe && L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
     return cudaSuccess;
 }

@@ -306,7 +306,10 @@ int dhara_get_krylov_traffic(dhara_handle *h, double *bytes, int64_t *iterations
  * result.  Defaults: tiles per domain, the most blocks per SM that fit,
  * overland resident when possible.  Results agree across schedules to
  * rounding (reductions run over tiles in a fixed order; a different tile
- * shape groups the sums differently), and bit for bit across block counts. */
+ * shape groups the sums differently), and bit for bit across block counts.
+ * Handles with few tiles per SM run the Krylov solve as a pipeline of one block
+ * per SM whatever the block count; a domain's results in such a handle and in a
+ * larger one agree to rounding. */
 typedef struct {
     int32_t krylov_blocks_per_sm;
     int32_t overland_resident;
@@ -319,7 +322,8 @@ typedef struct {
     double overland_ms;
     /* 1: each subsurface step is one persistent launch (prologue, every Picard
      * iteration's assembly, solve and check, epilogue) -- the default where
-     * that kernel runs as many blocks per SM as the Krylov kernel; 0: a launch
+     * that kernel runs as many blocks per SM as the Krylov kernel and the solve is
+     * not the pipeline; 0: a launch
      * per kernel (per-kernel timing then names every phase).  Results are the
      * same bit for bit. */
     int32_t fused_step;
