@@ -336,17 +336,23 @@ __device__ __forceinline__ void vg_eval<double>(double psi, double alpha_m, doub
     const double lambda = n - 1.0;
     const double m = lambda / n;
     const double _psi = psi * 100;
-    double _theta;
-    if (_psi < 0)
-        _theta = (theta_S - theta_R) / pow(1.0 + pow((alpha * (-_psi)), n), m) + theta_R;
-    else
-        _theta = theta_S;
+    // The reference evaluates each of these powers where it needs it; here each is
+    // taken once (six of them, the same values).  A saturated cell's are 1 and 0.
+    if (!(_psi < 0) && m > 0.0 && theta_S > theta_R) {
+        theta = theta_S;
+        K = Ksat;
+        C = 0.0;
+        return;
+    }
+    const double ax = alpha * fabs(_psi);
+    const double axn = pow(ax, n), u = 1.0 + axn;
+    const double _theta = _psi < 0 ? (theta_S - theta_R) / pow(u, m) + theta_R : theta_S;
     theta = _theta;
     const double Se = (_theta - theta_R) / (theta_S - theta_R);
-    K = Ksat * sqrt(Se) * (1.0 - pow(1.0 - pow(Se, 1.0 / m), m)) * (1.0 - pow(1.0 - pow(Se, 1.0 / m), m));
+    const double f = 1.0 - pow(1.0 - pow(Se, 1.0 / m), m);
+    K = Ksat * sqrt(Se) * f * f;
     if (_psi < 0)
-        C = 100 * alpha * n * (1.0 / n - 1.0) * pow(alpha * fabs(_psi), n - 1) * (theta_R - theta_S) *
-            pow(pow(alpha * fabs(_psi), n) + 1, 1.0 / n - 2.0);
+        C = 100 * alpha * n * (1.0 / n - 1.0) * pow(ax, n - 1) * (theta_R - theta_S) * pow(u, 1.0 / n - 2.0);
     else
         C = 0.0;
 }
@@ -423,8 +429,8 @@ struct ColumnRef {
     bool valid;
 };
 
-template <int G = 1>
-__device__ __forceinline__ ColumnRef column_of(const DevPtrs &P, int tile) {
+// Column `th` of a tile's TILE_THREADS.
+__device__ __forceinline__ ColumnRef column_at(const DevPtrs &P, int tile, int th) {
     const TileDesc t = P.tiles[tile];
     const DomainDesc &D = P.dom[t.dom];
     ColumnRef r;
@@ -432,8 +438,8 @@ __device__ __forceinline__ ColumnRef column_of(const DevPtrs &P, int tile) {
     r.tx = D.tx;
     r.ty = D.ty;
     r.tx_log2 = D.tx_log2;
-    r.i = t.x0 + (tile_thread<G>() & (D.tx - 1));
-    r.j = t.y0 + (tile_thread<G>() >> D.tx_log2);
+    r.i = t.x0 + (th & (D.tx - 1));
+    r.j = t.y0 + (th >> D.tx_log2);
     r.nx = D.nx;
     r.ny = D.ny;
     r.nz = D.nz;
@@ -443,4 +449,9 @@ __device__ __forceinline__ ColumnRef column_of(const DevPtrs &P, int tile) {
     r.g0 = D.off3 + (long long)r.j * D.nxp + r.i;
     r.c = D.off2 + (long long)r.j * D.nx + r.i;
     return r;
+}
+// The thread's column.
+template <int G = 1>
+__device__ __forceinline__ ColumnRef column_of(const DevPtrs &P, int tile) {
+    return column_at(P, tile, tile_thread<G>());
 }

@@ -192,26 +192,21 @@ __global__ void k_prologue(DevPtrs P) {
 }
 
 // -------------------------------------------------------------- assembly
-// One thread per column marching k = 0..nz-1 with K of k-1, k, k+1 in
-// registers.  For Picard iteration m it forms psi^m (psi^n at m = 0, else the
-// reference's relaxation am*psi^m + (1-am)*psi^{m+1}), evaluates the closure
+// For Picard iteration m it forms psi^m (psi^n at m = 0, else the reference's
+// relaxation am*psi^m + (1-am)*psi^{m+1}), evaluates the closure
 // in T, and writes K (T), the storage diagonal D (T), the right-hand side b
 // (double) and psi^m (double).  The right-hand side is
 // SetUpRightHandSideSubsurface (src/subsurface.cu:106-122) plus the Neumann
 // terms of SetUpBoundaryConditionsSubsurface (126-353) in the reference's
 // order top, bottom, south, north, west, east; the bottom is free drainage
 // (q_b = K of the bottom cell, written to bcqb as the reference does).
-// Eight blocks per SM (64 registers): the FP64 closure's latency chains need the
-// warps more than the registers (measured 18 % faster than the uncapped 96).
-template <typename T, int G = 1>
-__device__ __forceinline__ void assemble_tile(const DevPtrs &P, int tile) {
+// The Krylov control of a solve, set by one thread per domain; whether the
+// domain's Picard iteration is still running.
+__device__ __forceinline__ bool assemble_begin(const DevPtrs &P, int tile, bool first_thread) {
     const TileDesc td = P.tiles[tile];
-    const DomainDesc &D = P.dom[td.dom];
-    const PicardCtrl &pc = P.pctrl[td.dom];
-    const int done = pc.done;
-    const int iter = pc.iter;
-    if (tile_thread<G>() == 0 && tile == 0) P.gctrl->kry_bar = 0;
-    if (tile_thread<G>() == 0 && tile == D.tile_begin) {
+    const int done = P.pctrl[td.dom].done;
+    if (first_thread && tile == 0) P.gctrl->kry_bar = 0;
+    if (first_thread && tile == P.dom[td.dom].tile_begin) {
         KrylovCtrl &kc = P.kctrl[td.dom];
         kc.active = done ? 0 : 1;
         kc.inner_active = 0;
@@ -223,83 +218,112 @@ __device__ __forceinline__ void assemble_tile(const DevPtrs &P, int tile) {
         kc.rho_last = 0.0;
         if (!done) atomicAdd(&P.gctrl->n_active, 1);
     }
-    if (done) return;
+    return !done;
+}
+
+// What a column's cells share.
+struct AssembleCol {
+    const ColumnRef &cr;
+    const DomainDesc &D;
+    double ssc, tr;      // Ss / (dt phi); transpiration
+    const double *root;  // root fractions
+    int iter;
+};
+__device__ __forceinline__ AssembleCol assemble_col(const DevPtrs &P, const DomainDesc &D, const ColumnRef &cr) {
+    const int proc = P.procmap[cr.c];
+    return AssembleCol{cr, D, D.Ss / D.dt / D.porosity, P.tr[cr.c],
+                       P.rda + (size_t)cr.dom * P.rda_stride + (size_t)proc * cr.nz, P.pctrl[cr.dom].iter};
+}
+__device__ __forceinline__ double assemble_psi(const DevPtrs &P, const DomainDesc &D, int iter, long long g) {
+    return (iter == 0) ? P.psin[g] : D.am * P.psim[g] + (1.0 - D.am) * P.x[g];
+}
+__device__ __forceinline__ void assemble_closure(const DevPtrs &P, const DomainDesc &D, long long g, double psi,
+                                                 double &th, double &K, double &C) {
+    const double a = D.has_alpha ? P.alpha[g] : D.alpha;
+    const double n = D.has_n ? P.nvg[g] : D.n;
+    closure(D, psi, a, n, P.ksat[g], th, K, C);
+}
+
+// Cell (column, k) = g from its psi^m and closure and K of the planes above and
+// below.
+template <typename T>
+__device__ __forceinline__ void assemble_cell(const DevPtrs &P, const AssembleCol &col, int k, long long g,
+                                              double psi_c, double thm, double K_c, double Cm, double K_up,
+                                              double K_n) {
+    const ColumnRef &cr = col.cr;
+    const DomainDesc &D = col.D;
+    const int nz = cr.nz;
+    const double dt = D.dt, dz = D.dz, dx = D.dx, dy = D.dy, ssc = col.ssc;
+    const double kd = (k == 0) ? 0.0 : 0.5 * (K_c + K_up);
+    const double ku = (k == nz - 1) ? 0.0 : 0.5 * (K_c + K_n);
+    double trodz = 0.0;
+    if (col.tr > 0) trodz = -col.tr * col.root[k] * D.sec / dz;
+    double rhs = ssc * thm * P.psin[g] + Cm / dt * psi_c - (ku - kd) / dz +
+                 (P.thetan[g] - thm) / dt + trodz / dt;
+    const double dz2inv = -1.0 / (dz * dz), dy2inv = -1.0 / (dy * dy), dx2inv = -1.0 / (dx * dx);
+    if (k == 0) rhs += (-P.qtop[cr.c] * dz) * dz2inv;
+    const long long bi = D.offWE + (long long)k * cr.ny + cr.j;
+    const long long bj = D.offSN + (long long)k * cr.nx + cr.i;
+    // Neumann terms only on non-Dirichlet faces (a Dirichlet face's rows are
+    // set by k_dir_fixed / k_dir_rows after this kernel)
+    const bool dd = D.has_dirichlet != 0;
+    if (k == nz - 1 && !(dd && P.dir_b[cr.c])) {
+        const double qb = K_c;
+        P.bcqb[cr.c] = qb;
+        rhs += (qb * dz) * dz2inv;
+    }
+    if (cr.j == 0 && !(dd && P.dir_s[bj])) rhs += (-P.bcqs[bj] * dy) * dy2inv;
+    if (cr.j == cr.ny - 1 && !(dd && P.dir_n[bj])) rhs += (P.bcqn[bj] * dy) * dy2inv;
+    if (cr.i == 0 && !(dd && P.dir_w[bi])) rhs += (-P.bcqw[bi] * dx) * dx2inv;
+    if (cr.i == cr.nx - 1 && !(dd && P.dir_e[bi])) rhs += (P.bcqe[bi] * dx) * dx2inv;
+
+    const double Dv = ssc * thm + Cm / dt;
+    P.K64[g] = K_c;
+    P.D64[g] = Dv;
+    if (!std::is_same<T, double>::value) {
+        ((T *)P.K)[g] = (T)K_c;
+        ((T *)P.D)[g] = (T)Dv;
+    }
+    P.b[g] = rhs;
+}
+
+// The saturation record (psi >= 0 switches the closure's branch) of a cell.
+__device__ __forceinline__ unsigned long long saturation_mix(const DevPtrs &P, int dom, int iter, long long g, double psi) {
+    return branch_mix(P.pctrl[dom].step * 64 + (iter & 63), BR_SATURATION, g, band3(psi, 0.0, 1e-9));
+}
+
+// One thread per column marching k = 0..nz-1 with K of k-1, k, k+1 in registers.
+template <typename T, int G = 1>
+__device__ __forceinline__ void assemble_tile(const DevPtrs &P, int tile) {
+    if (!assemble_begin(P, tile, tile_thread<G>() == 0)) return;
     const ColumnRef cr = column_of<G>(P, tile);
+    const DomainDesc &D = P.dom[cr.dom];
+    const int iter = P.pctrl[cr.dom].iter;
     if (records(D, BR_SATURATION)) {
-        // saturation (psi >= 0 switches the closure's branch) of every cell at psi^m
         unsigned long long bsig = 0;
         if (cr.valid) {
             long long g = cr.g0;
-            for (int k = 0; k < cr.nz; ++k, g += cr.sxy) {
-                const double psi = (iter == 0) ? P.psin[g] : D.am * P.psim[g] + (1.0 - D.am) * P.x[g];
-                bsig += branch_mix(pc.step * 64 + (iter & 63), BR_SATURATION, g, band3(psi, 0.0, 1e-9));
-            }
+            for (int k = 0; k < cr.nz; ++k, g += cr.sxy)
+                bsig += saturation_mix(P, cr.dom, iter, g, assemble_psi(P, D, iter, g));
         }
-        branch_commit(&P.diag[td.dom].branch_sig, bsig);
+        branch_commit(&P.diag[cr.dom].branch_sig, bsig);
     }
     if (!cr.valid) return;
     const int nz = cr.nz;
-    const double dt = D.dt, dz = D.dz, dx = D.dx, dy = D.dy;
-    const double am = D.am;
-    const double ssc = D.Ss / dt / D.porosity;
-    const double tr_col = P.tr[cr.c];
-    const int proc = P.procmap[cr.c];
-    const double *root = P.rda + (size_t)cr.dom * P.rda_stride + (size_t)proc * nz;
-
-    auto psi_m_at = [&](long long g) -> double {
-        return (iter == 0) ? P.psin[g] : am * P.psim[g] + (1.0 - am) * P.x[g];
-    };
-    auto eval = [&](long long g, double psi, double &th, double &Kv, double &Cv) {
-        const double a = D.has_alpha ? P.alpha[g] : D.alpha;
-        const double n = D.has_n ? P.nvg[g] : D.n;
-        closure(D, psi, a, n, P.ksat[g], th, Kv, Cv);
-    };
-
+    const AssembleCol col = assemble_col(P, D, cr);
     long long g = cr.g0;
-    double psi_c = psi_m_at(g);
+    double psi_c = assemble_psi(P, D, iter, g);
     double th_c, K_c, C_c;
-    eval(g, psi_c, th_c, K_c, C_c);
+    assemble_closure(P, D, g, psi_c, th_c, K_c, C_c);
     double K_up = 0.0;
     for (int k = 0; k < nz; ++k, g += cr.sxy) {
         double psi_n_nb = 0.0, th_n = 0.0, K_n = 0.0, C_n = 0.0;
         if (k + 1 < nz) {
-            psi_n_nb = psi_m_at(g + cr.sxy);
-            eval(g + cr.sxy, psi_n_nb, th_n, K_n, C_n);
+            psi_n_nb = assemble_psi(P, D, iter, g + cr.sxy);
+            assemble_closure(P, D, g + cr.sxy, psi_n_nb, th_n, K_n, C_n);
         }
-        const double kd = (k == 0) ? 0.0 : 0.5 * (K_c + K_up);
-        const double ku = (k == nz - 1) ? 0.0 : 0.5 * (K_c + K_n);
-        const double thm = th_c, Cm = C_c;
-        double trodz = 0.0;
-        if (tr_col > 0) trodz = -tr_col * root[k] * D.sec / dz;
-        double rhs = ssc * thm * P.psin[g] + Cm / dt * psi_c - (ku - kd) / dz +
-                     (P.thetan[g] - thm) / dt + trodz / dt;
-        const double dz2inv = -1.0 / (dz * dz), dy2inv = -1.0 / (dy * dy), dx2inv = -1.0 / (dx * dx);
-        if (k == 0) rhs += (-P.qtop[cr.c] * dz) * dz2inv;
-        const long long bi = D.offWE + (long long)k * cr.ny + cr.j;
-        const long long bj = D.offSN + (long long)k * cr.nx + cr.i;
-        // Neumann terms only on non-Dirichlet faces (a Dirichlet face's rows are
-        // set by k_dir_fixed / k_dir_rows after this kernel)
-        const bool dd = D.has_dirichlet != 0;
-        if (k == nz - 1 && !(dd && P.dir_b[cr.c])) {
-            const double qb = K_c;
-            P.bcqb[cr.c] = qb;
-            rhs += (qb * dz) * dz2inv;
-        }
-        if (cr.j == 0 && !(dd && P.dir_s[bj])) rhs += (-P.bcqs[bj] * dy) * dy2inv;
-        if (cr.j == cr.ny - 1 && !(dd && P.dir_n[bj])) rhs += (P.bcqn[bj] * dy) * dy2inv;
-        if (cr.i == 0 && !(dd && P.dir_w[bi])) rhs += (-P.bcqw[bi] * dx) * dx2inv;
-        if (cr.i == cr.nx - 1 && !(dd && P.dir_e[bi])) rhs += (P.bcqe[bi] * dx) * dx2inv;
-
-        const double Dv = ssc * thm + Cm / dt;
         P.psim[g] = psi_c;
-        P.K64[g] = K_c;
-        P.D64[g] = Dv;
-        if (!std::is_same<T, double>::value) {
-            ((T *)P.K)[g] = (T)K_c;
-            ((T *)P.D)[g] = (T)Dv;
-        }
-        P.b[g] = rhs;
-
+        assemble_cell<T>(P, col, k, g, psi_c, th_c, K_c, C_c, K_up, K_n);
         K_up = K_c;
         psi_c = psi_n_nb;
         th_c = th_n;
@@ -308,9 +332,46 @@ __device__ __forceinline__ void assemble_tile(const DevPtrs &P, int tile) {
     }
 }
 
+// Eight blocks per SM (64 registers): the FP64 closure's latency chains need the
+// warps more than the registers (measured 18 % faster than the uncapped 96).
 template <typename T>
 __global__ void __launch_bounds__(TILE_THREADS, 8) k_assemble(DevPtrs P) {
     assemble_tile<T>(P, blockIdx.x);
+}
+
+// The planes of a column in parallel: a block is 32 of a tile's columns, a warp
+// takes every blockDim.y-th plane of them.  The warps evaluate the closures of
+// their planes into shared memory; after a barrier, with K of the neighbouring
+// planes there, each finishes the same cells.
+#define ASSEMBLE_WARPS 32
+template <typename T>
+__global__ void __launch_bounds__(32 * ASSEMBLE_WARPS, 1) k_assemble_planes(DevPtrs P) {
+    extern __shared__ double s_cell[];  // K, theta, C of the 32 columns, plane by plane
+    const int tile = blockIdx.x / (TILE_THREADS / 32), lane = threadIdx.x, w = threadIdx.y, W = blockDim.y;
+    const int strip = blockIdx.x % (TILE_THREADS / 32);
+    if (!assemble_begin(P, tile, strip == 0 && lane == 0 && w == 0)) return;
+    const ColumnRef cr = column_at(P, tile, strip * 32 + lane);
+    const DomainDesc &D = P.dom[cr.dom];
+    const int nz = cr.nz, iter = P.pctrl[cr.dom].iter;
+    double *const sK = s_cell + lane, *const sth = sK + 32 * nz, *const sC = sth + 32 * nz;
+    unsigned long long bsig = 0;
+    if (cr.valid) {
+        long long g = cr.g0 + w * cr.sxy;
+        for (int k = w; k < nz; k += W, g += W * cr.sxy) {
+            const double psi = assemble_psi(P, D, iter, g);
+            assemble_closure(P, D, g, psi, sth[32 * k], sK[32 * k], sC[32 * k]);
+            P.psim[g] = psi;
+            if (records(D, BR_SATURATION)) bsig += saturation_mix(P, cr.dom, iter, g, psi);
+        }
+    }
+    if (records(D, BR_SATURATION)) branch_commit(&P.diag[cr.dom].branch_sig, bsig);
+    __syncthreads();
+    if (!cr.valid) return;
+    const AssembleCol col = assemble_col(P, D, cr);
+    long long g = cr.g0 + w * cr.sxy;
+    for (int k = w; k < nz; k += W, g += W * cr.sxy)
+        assemble_cell<T>(P, col, k, g, P.psim[g], sth[32 * k], sK[32 * k], sC[32 * k], k > 0 ? sK[32 * (k - 1)] : 0.0,
+                         k + 1 < nz ? sK[32 * (k + 1)] : 0.0);
 }
 
 // ---------------------------------------------------------- Dirichlet faces
@@ -395,16 +456,17 @@ __device__ __forceinline__ bool dir_rules(const ColumnRef &cr, int k, const DirF
     return fixed;
 }
 
-// Pass 1: identity rows (D = -1, x = b = the row's right-hand side).
+// Pass 1: identity rows (D = -1, x = b = the row's right-hand side).  Every dk-th
+// plane from k0 on.
 template <typename T, int G = 1>
-__device__ __forceinline__ void dir_fixed_tile(const DevPtrs &P, int tile) {
+__device__ __forceinline__ void dir_fixed_tile(const DevPtrs &P, int tile, int k0 = 0, int dk = 1) {
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
     if (!D.has_dirichlet || P.pctrl[td.dom].done) return;
     const ColumnRef cr = column_of<G>(P, tile);
     if (!cr.valid) return;
-    long long g = cr.g0;
-    for (int k = 0; k < cr.nz; ++k, g += cr.sxy) {
+    long long g = cr.g0 + k0 * cr.sxy;
+    for (int k = k0; k < cr.nz; k += dk, g += dk * cr.sxy) {
         const DirFaces f = dir_faces(P, D, cr, k);
         if (!(f.b || f.s || f.n || f.w || f.e)) continue;
         double v = P.b[g];
@@ -418,21 +480,21 @@ __device__ __forceinline__ void dir_fixed_tile(const DevPtrs &P, int tile) {
 
 template <typename T>
 __global__ void __launch_bounds__(TILE_THREADS) k_dir_fixed(DevPtrs P) {
-    dir_fixed_tile<T>(P, blockIdx.x);
+    dir_fixed_tile<T>(P, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // Pass 2: the rows next to identity rows get the reference's elimination
 // terms, less the coupling the matrix-free stencil applies to the fixed value.
 template <typename T, int G = 1>
-__device__ __forceinline__ void dir_rows_tile(const DevPtrs &P, int tile) {
+__device__ __forceinline__ void dir_rows_tile(const DevPtrs &P, int tile, int k0 = 0, int dk = 1) {
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
     if (!D.has_dirichlet || P.pctrl[td.dom].done) return;
     const ColumnRef cr = column_of<G>(P, tile);
     if (!cr.valid) return;
     const double ix2 = 1.0 / (D.dx * D.dx), iy2 = 1.0 / (D.dy * D.dy), iz2 = 1.0 / (D.dz * D.dz);
-    long long g = cr.g0;
-    for (int k = 0; k < cr.nz; ++k, g += cr.sxy) {
+    long long g = cr.g0 + k0 * cr.sxy;
+    for (int k = k0; k < cr.nz; k += dk, g += dk * cr.sxy) {
         if (P.D64[g] < 0.0) continue;  // identity row
         const DirFaces f = dir_faces(P, D, cr, k);
         if (!(f.b || f.s || f.n || f.w || f.e)) continue;
@@ -450,7 +512,7 @@ __device__ __forceinline__ void dir_rows_tile(const DevPtrs &P, int tile) {
 
 template <typename T>
 __global__ void __launch_bounds__(TILE_THREADS) k_dir_rows(DevPtrs P) {
-    dir_rows_tile<T>(P, blockIdx.x);
+    dir_rows_tile<T>(P, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // ------------------------------------------------------------ Krylov solve
@@ -1217,23 +1279,37 @@ __device__ __forceinline__ void picard_check_tile(const DevPtrs &P, int tile) {
     double mx = 0.0;
     int nonfinite = 0;
     if (cr.valid) {
-        long long g = cr.g0;
-        for (int k = 0; k < cr.nz; ++k, g += cr.sxy) {
-            const double xn = P.x[g], xm = P.psim[g];
-            double d;
-            if (D.picard_rule == DHARA_PICARD_THETA_RELATIVE) {
-                const double a = D.has_alpha ? P.alpha[g] : D.alpha;
-                const double n = D.has_n ? P.nvg[g] : D.n;
-                const double t1 = vg_theta(xn, a, n, D.theta_s, D.theta_r);
-                const double t0 = vg_theta(xm, a, n, D.theta_s, D.theta_r);
-                d = fabs((t1 - t0) / t1);
-            } else if (D.picard_rule == DHARA_PICARD_PSI_ABSOLUTE) {
-                d = fabs(xn - xm);
-            } else {
-                d = fabs((xn - xm) / xn);
+        // the loads of CHECK_BATCH planes together: one after the other they cost
+        // their latency per plane (128x128x30, ten checks: 0.21 ms, so 0.14; 1024x1024x40 2.04 / 1.53)
+        constexpr int CHECK_BATCH = 8;
+        for (int k0 = 0; k0 < cr.nz; k0 += CHECK_BATCH) {
+            double bn[CHECK_BATCH], bm[CHECK_BATCH];
+#pragma unroll
+            for (int e = 0; e < CHECK_BATCH; ++e) {
+                const long long g = cr.g0 + (long long)(k0 + e < cr.nz ? k0 + e : k0) * cr.sxy;
+                bn[e] = P.x[g];
+                bm[e] = P.psim[g];
             }
-            if (!(d == d)) { nonfinite = 1; d = INFINITY; }
-            mx = fmax(mx, d);
+#pragma unroll
+            for (int e = 0; e < CHECK_BATCH; ++e) {
+                if (k0 + e >= cr.nz) break;
+                const double xn = bn[e], xm = bm[e];
+                double d;
+                if (D.picard_rule == DHARA_PICARD_THETA_RELATIVE) {
+                    const long long g = cr.g0 + (long long)(k0 + e) * cr.sxy;
+                    const double a = D.has_alpha ? P.alpha[g] : D.alpha;
+                    const double n = D.has_n ? P.nvg[g] : D.n;
+                    const double t1 = vg_theta(xn, a, n, D.theta_s, D.theta_r);
+                    const double t0 = vg_theta(xm, a, n, D.theta_s, D.theta_r);
+                    d = fabs((t1 - t0) / t1);
+                } else if (D.picard_rule == DHARA_PICARD_PSI_ABSOLUTE) {
+                    d = fabs(xn - xm);
+                } else {
+                    d = fabs((xn - xm) / xn);
+                }
+                if (!(d == d)) { nonfinite = 1; d = INFINITY; }
+                mx = fmax(mx, d);
+            }
         }
     }
     if (nonfinite) atomicOr(&P.diag[td.dom].nonfinite, 1);
@@ -1525,7 +1601,22 @@ cudaError_t launch_prepare(const DevPtrs &P, int mixed, cudaStream_t s) {
 }
 
 cudaError_t launch_assemble(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s) {
-    if (L.mixed) k_assemble<float><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
+    // Planes in parallel while marching leaves the chip idle -- one wave of eight
+    // blocks per SM, or few of them -- or the closure's latency bounds it.  Ten
+    // assemblies, marching / planes in ms: 128x128x30 0.83 / 0.30, 388x388x40 3.41 /
+    // 2.45, 512x512x40 (14 tiles per SM) 4.01 / 3.90, 640x640x40 (22) 5.89 / 6.00, 256
+    // domains (79) 15.5 / 17.8; FP64 32x32x20 1.11 / 0.15, 388x388x40 5.68 / 4.24,
+    // 512x512x40 7.83 / 7.16, 768x768x40 (32) 17.7 / 16.9.  A warp per plane (32 at
+    // most) while each SM has one block (32x32x20 FP64, 16 warps 0.21), else eight
+    // (301x211x33, 16 / 8 warps 1.23 / 1.08).
+    if (P.ntiles <= (L.mixed ? 16 : 32) * L.sms) {
+        const int strips = P.ntiles * (TILE_THREADS / 32);
+        const int most = strips <= L.sms ? ASSEMBLE_WARPS : 8;
+        const dim3 block(32, L.nz_max < most ? L.nz_max : most);
+        const int smem = 3 * 32 * L.nz_max * (int)sizeof(double);
+        if (L.mixed) k_assemble_planes<float><<<strips, block, smem, s>>>(P);
+        else k_assemble_planes<double><<<strips, block, smem, s>>>(P);
+    } else if (L.mixed) k_assemble<float><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
     else k_assemble<double><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
     return cudaGetLastError();
 }
@@ -1537,12 +1628,16 @@ cudaError_t launch_epilogue(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s
 }
 
 cudaError_t launch_dirichlet(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s) {
+    // the planes of a tile by as many blocks as fill the chip: a plane costs a
+    // chain of loads (53x37x21 FP64, ten of both passes: 0.67 ms marching, 0.16 so)
+    const int want = 16 * L.sms / P.ntiles;
+    const dim3 grid(P.ntiles, want < 1 ? 1 : want < L.nz_max ? want : L.nz_max);
     if (L.mixed) {
-        k_dir_fixed<float><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
-        k_dir_rows<float><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
+        k_dir_fixed<float><<<grid, TILE_THREADS, 0, s>>>(P);
+        k_dir_rows<float><<<grid, TILE_THREADS, 0, s>>>(P);
     } else {
-        k_dir_fixed<double><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
-        k_dir_rows<double><<<P.ntiles, TILE_THREADS, 0, s>>>(P);
+        k_dir_fixed<double><<<grid, TILE_THREADS, 0, s>>>(P);
+        k_dir_rows<double><<<grid, TILE_THREADS, 0, s>>>(P);
     }
     return cudaGetLastError();
 }
