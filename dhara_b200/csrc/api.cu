@@ -781,9 +781,11 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
     std::vector<MgDom> mgd;
     std::vector<MgChunk> mgc;
     int lchunk[MG_MAXLEV + 2];
-    int mg_lg = 0;
+    int mg_lg = 0, sms = 1;
     long long mg_nc = 0, mg_npw = 0, mg_ndinv = 0;
-    if (!mg_plan(h->hdom, mgd, mgc, lchunk, mg_lg, mg_nc, mg_npw, mg_ndinv))
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        return bail(fail(DHARA_ERR_CUDA, "cannot read the device's properties"));
+    if (!mg_plan(h->hdom, mgd, mgc, lchunk, mg_lg, mg_nc, mg_npw, mg_ndinv, sms, P.mg_size0))
         return bail(fail(DHARA_ERR_UNSUPPORTED, "a surface grid needs more than %d multigrid levels", MG_MAXLEV));
     MgDom *d_mgd = nullptr;
     MgChunk *d_mgc = nullptr;

@@ -202,9 +202,10 @@ struct OlfSegState {
 // their operators (5), smoother weights, vectors b, x, t and interpolation
 // weights (4 floats) per point, and the coarsest level's inverse
 #define MG_SMEM_BYTES ((MG_SMEM_PTS * 11 + MG_DENSE_PTS * MG_DENSE_PTS) * 8)
-#ifndef MG_CHUNK0
-#define MG_CHUNK0 (4 * OLF_THREADS)  // points of a level-0 chunk (the CG's vectors), four per thread
-#endif
+#define MG_THREADS 512
+// Level 0 (the CG's vectors) is summed by groups of MG_THREADS consecutive points
+// of a domain and worked on in chunks of 1, 2 or 4 groups, a point of each per thread.
+#define MG_CHUNK0 4
 struct MgDom {
     int nlev;                      // levels; 0 when the domain has no interior cell
     int lc;                        // first level run by the domain's block (levels lc .. nlev-1)
@@ -217,7 +218,7 @@ struct MgDom {
     long long pwo[MG_MAXLEV];      // first interpolation-weight slot of level l (l < nlev - 1)
     long long dio;                 // first entry of the coarsest level's inverse
 };
-// A run of up to OLF_THREADS (level 0: MG_CHUNK0) consecutive points of one
+// A run of up to MG_THREADS (level 0: mg_size0 groups of them) consecutive points of one
 // level of one domain.
 struct MgChunk {
     int dom, lev, first, count;
@@ -289,6 +290,7 @@ struct DevPtrs {
     const MgChunk *mgc;  // chunk lists: level l's at mg_lchunk[l] .. mg_lchunk[l+1]-1
     int mg_lchunk[MG_MAXLEV + 2];
     int mg_lg;           // levels run as grid phases: the largest lc of any domain
+    int mg_size0;        // groups of a level-0 chunk
     int mg_nchunk0;      // level-0 chunks (every domain with an interior)
     int n_frozen;        // domains with DomainDesc::frozen set (time-step halving)
     long long mg_nc;     // coarse points of all domains and levels
@@ -374,7 +376,7 @@ cudaError_t launch_overland_finish(const DevPtrs &P, long long ctot, cudaStream_
 // levels, the chunk lists (level by level) and the number of coarse points.
 cudaError_t launch_overland_mg(const DevPtrs &P, const LaunchCfg &L, long long ctot, cudaStream_t s);
 bool mg_plan(const std::vector<DomainDesc> &doms, std::vector<MgDom> &mgd, std::vector<MgChunk> &chunks,
-             int (&lchunk)[MG_MAXLEV + 2], int &lg, long long &nc, long long &npw, long long &ndinv);
+             int (&lchunk)[MG_MAXLEV + 2], int &lg, long long &nc, long long &npw, long long &ndinv, int blocks, int &size0);
 cudaError_t configure_mg(LaunchCfg &L, int device);
 // Discrete adjoint (adjoint.cu).  Tape of one checkpoint segment, the
 // carried adjoint state and the gradient accumulators; 3D arrays in the

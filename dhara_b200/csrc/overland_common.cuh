@@ -10,9 +10,9 @@ __device__ __forceinline__ bool is_ring(int i, int j, int nx, int ny) {
     return i == 0 || j == 0 || i == nx - 1 || j == ny - 1;
 }
 
-template <int NV>
+template <int NV, int THREADS = OLF_THREADS>
 __device__ __forceinline__ void olf_block_sum(double (&v)[NV]) {
-    __shared__ double s_w[NV][OLF_THREADS / 32];
+    __shared__ double s_w[NV][THREADS / 32];
     __shared__ double s_out[NV];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -26,7 +26,7 @@ __device__ __forceinline__ void olf_block_sum(double (&v)[NV]) {
     if (threadIdx.x < NV) {
         double a = 0.0;
 #pragma unroll
-        for (int w = 0; w < OLF_THREADS / 32; ++w) a += s_w[threadIdx.x][w];
+        for (int w = 0; w < THREADS / 32; ++w) a += s_w[threadIdx.x][w];
         s_out[threadIdx.x] = a;
     }
     __syncthreads();

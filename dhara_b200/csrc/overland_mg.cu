@@ -45,18 +45,24 @@
 // domain's coarsest levels, as many as fit MG_SMEM_PTS points together, run
 // in one block out of shared memory with block barriers, their operators set
 // up there and kept for the whole solve when the block owns one domain; the
-// finer ones run as grid phases, level 0 in chunks of MG_CHUNK0 points (four
-// per thread) and the others one point per thread.  The pre-smoothing and
+// finer ones run as grid phases, level 0 in chunks of one, two or four points per
+// thread (mg_plan) and the others one point per thread.  The pre-smoothing and
 // the residual are folded into a stored 5 x 5 restriction stencil per coarse
 // point (P^T (I - A W^-1), formed at set-up), and the prolongation is fused
 // into the post-smoothing (each point recomputes the few neighbour values it
 // needs), so a grid level costs one barrier on the way down and one on the
 // way up; with q = A z + beta q
 // the CG forms p and q in one phase.  An iteration with L grid levels is
-// 2 L + 3 barriers (eleven on a 512 x 512 surface).  Every reduction runs over
+// 2 L + 3 barriers (eleven on a 512 x 512 surface).  What bounds it is latency:
+// barriers, the chains of L2 reads after each (one domain's descriptors are kept in
+// shared memory), and the block levels' serial phases.  512 threads a block and one
+// point of the small levels' each (256 threads and two blocks per SM had half the
+// threads there): a solve of 61x47 0.84 to 0.62 ms, 53x37 0.84 to 0.65, 128x128 1.30
+// to 1.13, 512x512 2.82 to 2.29.  Every reduction runs over
 // chunks in a fixed order, so results do not depend on the block count.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "overland_common.cuh"
 
@@ -557,6 +563,7 @@ __device__ __forceinline__ SmemMG smem_mg(double *base) {
 
 struct SL {
     int m, n, o;  // points and first slot of the level
+    float im;     // 1 / m
     __device__ __forceinline__ int at(int i, int j) const { return o + j * m + i; }
 };
 
@@ -587,26 +594,69 @@ __device__ __forceinline__ double s_apply(const Row9 &r, const double *x, const 
     return s;
 }
 
+// Point p of a level: p / m from the reciprocal, exact for p < MG_SMEM_PTS (the
+// error of (p + 1/2) / m is far below its distance to a whole number, 1 / 2m).
+__device__ __forceinline__ void s_point(const SL &v, int p, int &i, int &j) {
+    j = (int)(((float)p + 0.5f) * v.im);
+    i = p - j * v.m;
+}
 template <typename Fn>
 __device__ __forceinline__ void s_points(const SL &v, Fn fn) {
     const int tot = v.m * v.n;
-    for (int p = threadIdx.x; p < tot; p += blockDim.x) fn(p % v.m, p / v.m);
+    for (int p = threadIdx.x; p < tot; p += MG_THREADS) {
+        int i, j;
+        s_point(v, p, i, j);
+        fn(i, j);
+    }
+}
+// put(slot, value(i, j)) at every point of a level: a thread's points (all of them
+// up to MG_SMEM_PTS) are evaluated together and stored afterwards, since the
+// compiler may not move a point's loads across an earlier point's store.
+template <int M, typename Val, typename Put>
+__device__ __forceinline__ void s_batch(const SL &v, int tot, Val value, Put put) {
+    double r[M];
+#pragma unroll
+    for (int e = 0; e < M; ++e) {
+        const int p = (int)threadIdx.x + e * MG_THREADS;
+        int i, j;
+        s_point(v, p < tot ? p : 0, i, j);
+        r[e] = value(i, j);
+    }
+#pragma unroll
+    for (int e = 0; e < M; ++e) {
+        const int p = (int)threadIdx.x + e * MG_THREADS;
+        if (p < tot) put(v.o + p, r[e]);
+    }
+}
+template <typename Val, typename Put>
+__device__ __forceinline__ void s_eval(const SL &v, Val value, Put put) {
+    const int tot = v.m * v.n, warp0 = (int)threadIdx.x & ~31;
+    static_assert(MG_SMEM_PTS <= 3 * MG_THREADS, "points of a level per thread");
+    if (warp0 >= tot) return;
+    if (warp0 + MG_THREADS >= tot) s_batch<1>(v, tot, value, put);
+    else if (warp0 + 2 * MG_THREADS >= tot) s_batch<2>(v, tot, value, put);
+    else s_batch<3>(v, tot, value, put);
 }
 
-// Levels lc .. nlev-1 packed in shared memory.
-__device__ __forceinline__ void s_levels(const MgDom &g, SL (&lv)[MG_MAXLEV]) {
-    int o = 0;
-    for (int l = g.lc; l < g.nlev; ++l) {
-        lv[l] = SL{g.m[l], g.n[l], o};
-        o += g.m[l] * g.n[l];
+// Levels lc .. nlev-1 packed in shared memory, the table of them too (indexed at
+// run time it would be in local memory: 61x47 0.645 / 0.62 ms).  All threads call it.
+__device__ __forceinline__ void s_levels(const MgDom &g, SL *lv) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int o = 0;
+        for (int l = g.lc; l < g.nlev; ++l) {
+            lv[l] = SL{g.m[l], g.n[l], o, 1.0f / (float)g.m[l]};
+            o += g.m[l] * g.n[l];
+        }
     }
+    __syncthreads();
 }
 
 // Level lc's operator into shared memory (level 0: from the conductances)
 // with, when `all`, the coarser operators, the smoother and interpolation
 // weights and the coarsest inverse that the set-up left in global memory.
 __device__ void block_load(const DevPtrs &P, const DomainDesc &D, long long ctot, const MgDom &g, const SmemMG &S,
-                           const SL (&lv)[MG_MAXLEV], bool all) {
+                           const SL *lv, bool all) {
     const int last = all ? g.nlev - 1 : g.lc;
     for (int l = g.lc; l <= last; ++l) {
         const SL v = lv[l];
@@ -682,7 +732,7 @@ __device__ void dense_inverse(const SmemMG &S, const SL &v, double *M, double *d
 // global memory for a block that must reload them.
 __device__ void block_setup(const DevPtrs &P, const DomainDesc &D, long long ctot, const MgDom &g, double *smem) {
     const SmemMG S = smem_mg(smem);
-    SL lv[MG_MAXLEV];
+    __shared__ SL lv[MG_MAXLEV];
     s_levels(g, lv);
     block_load(P, D, ctot, g, S, lv, false);
     for (int l = g.lc; l + 1 < g.nlev; ++l) {
@@ -726,7 +776,7 @@ __device__ void block_setup(const DevPtrs &P, const DomainDesc &D, long long cto
 __device__ void block_vcycle(const DevPtrs &P, const DomainDesc &D, long long ctot, const MgDom &g, int dom,
                              double *smem, int &resident) {
     const SmemMG S = smem_mg(smem);
-    SL lv[MG_MAXLEV];
+    __shared__ SL lv[MG_MAXLEV];
     s_levels(g, lv);
     const bool reload = resident != dom;
     __syncthreads();  // every thread has read `resident`
@@ -749,9 +799,10 @@ __device__ void block_vcycle(const DevPtrs &P, const DomainDesc &D, long long ct
         const SL f = lv[l], c = lv[l + 1];
         const bool hx = g.hx[l], hy = g.hy[l];
         __syncthreads();
-        s_points(f, [&](int i, int j) { S.t[f.at(i, j)] = S.b[f.at(i, j)] - s_apply(s_row(S, f, i, j), S.x, f, i, j); });
+        s_eval(f, [&](int i, int j) { return S.b[f.at(i, j)] - s_apply(s_row(S, f, i, j), S.x, f, i, j); },
+               [&](int q, double t) { S.t[q] = t; });
         __syncthreads();
-        s_points(c, [&](int I, int J) {
+        s_eval(c, [&](int I, int J) {
             double acc = 0.0;
 #pragma unroll
             for (int bb = 0; bb < 3; ++bb)
@@ -764,7 +815,8 @@ __device__ void block_vcycle(const DevPtrs &P, const DomainDesc &D, long long ct
                     if (vx != 0.0 && vy != 0.0)
                         acc += slot(S.pw[f.at(fx, fy)], child_slot(aa, hx) + 2 * child_slot(bb, hy)) * S.t[f.at(fx, fy)];
                 }
-            const int q = c.at(I, J);
+            return acc;
+        }, [&](int q, double acc) {
             S.b[q] = acc;
             if (l + 1 < L) S.x[q] = S.w[q] * acc;
         });
@@ -785,7 +837,7 @@ __device__ void block_vcycle(const DevPtrs &P, const DomainDesc &D, long long ct
         const SL f = lv[l], c = lv[l + 1];
         const bool hx = g.hx[l], hy = g.hy[l];
         __syncthreads();
-        s_points(f, [&](int i, int j) {
+        s_eval(f, [&](int i, int j) {
             int px0, px1, py0, py1;
             double ux0, ux1, uy0, uy1;
             parents2(i, hx, c.m, px0, ux0, px1, ux1);
@@ -796,13 +848,13 @@ __device__ void block_vcycle(const DevPtrs &P, const DomainDesc &D, long long ct
             if (ux1 != 0.0 && uy0 != 0.0) sum += (double)w.y * S.t[c.at(px1, py0)];
             if (ux0 != 0.0 && uy1 != 0.0) sum += (double)w.z * S.t[c.at(px0, py1)];
             if (ux1 != 0.0 && uy1 != 0.0) sum += (double)w.w * S.t[c.at(px1, py1)];
-            S.x[f.at(i, j)] += sum;
-        });
+            return S.x[f.at(i, j)] + sum;
+        }, [&](int q, double x) { S.x[q] = x; });
         __syncthreads();
-        s_points(f, [&](int i, int j) {
+        s_eval(f, [&](int i, int j) {
             const int q = f.at(i, j);
-            S.t[q] = S.x[q] + S.w[q] * (S.b[q] - s_apply(s_row(S, f, i, j), S.x, f, i, j));
-        });
+            return S.x[q] + S.w[q] * (S.b[q] - s_apply(s_row(S, f, i, j), S.x, f, i, j));
+        }, [&](int q, double t) { S.t[q] = t; });
     }
     __syncthreads();
     // ---- level lc's result
@@ -817,18 +869,34 @@ __device__ void block_vcycle(const DevPtrs &P, const DomainDesc &D, long long ct
 
 // ------------------------------------------------------------ domain sums
 // Sums of the given chunk-partial slots over the domain's level-0 chunks,
-// taken by each warp on its own (lane k sums chunks k, k+32, ..., then a
-// butterfly), so every warp of every block gets the same bits with no block
-// barrier.
+// taken by each warp on its own (lane k sums the sets k, k+32, ... of MG_CHUNK0
+// groups, then a butterfly), so every warp of every block gets the same bits with
+// no block barrier.  A set is a chunk, or two or four chunks added in pairs, so
+// the bits do not depend on the chunks' size either.
 template <int NV>
 __device__ __forceinline__ void chunk_sums(const DevPtrs &P, const MgDom &g, const int (&slot)[NV], double (&v)[NV]) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, per = MG_CHUNK0 / P.mg_size0;
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = 0.0;
+    const double *part = P.mg_part + g.c0_first;
+    const size_t stride = P.mg_nchunk0;
+    if (per == 1) {
 #pragma unroll 8
-    for (int k = lane; k < g.c0_count; k += 32) {
+        for (int k = lane; k < g.c0_count; k += 32) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) v[i] += __ldcg(&P.mg_part[(size_t)slot[i] * P.mg_nchunk0 + g.c0_first + k]);
+            for (int i = 0; i < NV; ++i) v[i] += __ldcg(part + slot[i] * stride + k);
+        }
+    } else {
+        for (int k = lane * per; k < g.c0_count; k += 32 * per) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                double q[MG_CHUNK0];
+#pragma unroll
+                for (int e = 0; e < MG_CHUNK0; ++e)
+                    q[e] = e < per && k + e < g.c0_count ? __ldcg(part + slot[i] * stride + k + e) : 0.0;
+                v[i] += (q[0] + q[1]) + (q[2] + q[3]);
+            }
+        }
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i)
@@ -860,15 +928,36 @@ __device__ __forceinline__ DomSums decision_sums(const DevPtrs &P, const MgDom &
 }  // namespace
 
 // --------------------------------------------------------------- the solve
-__global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long long ctot) {
+__global__ void __launch_bounds__(MG_THREADS, 1) k_olf_mgcg(DevPtrs P, long long ctot) {
     extern __shared__ double s_mg[];  // a domain's block levels (block_vcycle)
     __shared__ int s_resident;        // the domain whose block levels are set up in s_mg
+    // one domain's descriptors are kept here: after a barrier L1 holds nothing, and
+    // reading them again is a chain of L2 round trips in every phase
+    __shared__ MgDom s_g;
+    __shared__ DomainDesc s_D;
     const int tid = threadIdx.x;
     if (tid == 0) s_resident = -1;
+    const bool one = P.ndom == 1;
+    if (one) {
+        static_assert(sizeof(MgDom) % 4 == 0 && sizeof(DomainDesc) % 4 == 0, "copied in words");
+        for (int w = tid; w < (int)(sizeof(MgDom) / 4); w += MG_THREADS) ((int *)&s_g)[w] = ((const int *)P.mgd)[w];
+        for (int w = tid; w < (int)(sizeof(DomainDesc) / 4); w += MG_THREADS) ((int *)&s_D)[w] = ((const int *)P.dom)[w];
+        __syncthreads();
+    }
+    auto mgd = [&](int d) -> const MgDom & { return one ? s_g : P.mgd[d]; };
+    auto dom = [&](int d) -> const DomainDesc & { return one ? s_D : P.dom[d]; };
     // barrier: one counter that every block adds to once per phase (zeroed by
     // k_olf_setup before every solve)
     unsigned int epoch = 0;
-    auto sync = [&]() { return counter_sync(&P.gctrl->olf_bar, (++epoch) * gridDim.x, P.barrier); };
+    // (a single block meets itself; the fence orders its writes for its L2 reads)
+    auto sync = [&]() {
+        if (gridDim.x == 1) {
+            __threadfence();
+            __syncthreads();
+            return true;
+        }
+        return counter_sync(&P.gctrl->olf_bar, (++epoch) * gridDim.x, P.barrier);
+    };
     const int Lg = P.mg_lg;
     const int nchunk0 = P.mg_nchunk0;
     double *part = P.mg_part;
@@ -876,8 +965,14 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
     // chunks of level l, block-strided; fn(chunk, MgDom, DomainDesc)
     auto chunks = [&](int l, auto fn) {
         for (int k = P.mg_lchunk[l] + blockIdx.x; k < P.mg_lchunk[l + 1]; k += gridDim.x) {
-            const MgChunk ch = P.mgc[k];
-            fn(k, ch, P.mgd[ch.dom], P.dom[ch.dom]);
+            if (one) {
+                const int size = l == 0 ? P.mg_size0 * MG_THREADS : MG_THREADS, first = (k - P.mg_lchunk[l]) * size;
+                const int left = s_g.m[l] * s_g.n[l] - first;
+                fn(k, MgChunk{0, l, first, left < size ? left : size}, s_g, s_D);
+            } else {
+                const MgChunk ch = P.mgc[k];
+                fn(k, ch, P.mgd[ch.dom], P.dom[ch.dom]);
+            }
         }
     };
     auto point_of = [&](const MgChunk &ch, const MgDom &g, int &i, int &j) {
@@ -887,33 +982,49 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
         j = p / g.m[ch.lev];
         return true;
     };
-    // the points of a level-0 chunk (MG_CHUNK0 = 4 per thread)
-    auto points0 = [&](const MgChunk &ch, const MgDom &g, auto fn) {
-#pragma unroll
-        for (int q = 0; q < MG_CHUNK0 / OLF_THREADS; ++q) {
-            const int o = tid + q * OLF_THREADS;
-            if (o < ch.count) {
-                const int p = ch.first + o;
-                fn(p % g.m[0], p / g.m[0]);
-            }
+    // Level 0: fn(NQ, chunk, MgDom, DomainDesc) with the chunk's groups as a constant
+    auto chunks0 = [&](auto fn) {
+        chunks(0, [&](int, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
+            if (ch.count <= MG_THREADS) fn(std::integral_constant<int, 1>{}, ch, g, D);
+            else if (ch.count <= 2 * MG_THREADS) fn(std::integral_constant<int, 2>{}, ch, g, D);
+            else fn(std::integral_constant<int, MG_CHUNK0>{}, ch, g, D);
+        });
+    };
+    // a chunk's sums into partials `slot`: by group, then these in pairs (chunk_sums
+    // goes on in the same order where a chunk has fewer groups)
+    auto group_sums = [&](int slot, auto &v, const MgChunk &ch, const MgDom &g) {
+        constexpr int NQ = (int)(sizeof(v) / sizeof(double));
+        olf_block_sum<NQ, MG_THREADS>(v);
+        if (tid == 0) {
+            double a = v[0];
+            if constexpr (NQ == 2) a = v[0] + v[1];
+            if constexpr (NQ == 4) a = (v[0] + v[1]) + (v[2] + v[3]);
+            pslot(slot, g.c0_first + ch.first / (P.mg_size0 * MG_THREADS)) = a;
         }
     };
-    auto active = [&](int d) { return __ldcg(&P.mgctl[d].active) != 0; };
+    // one domain: the loop ends with it
+    const bool alive = one && s_g.nlev > 0 && !s_D.frozen;
+    auto active = [&](int d) { return one ? alive : __ldcg(&P.mgctl[d].active) != 0; };
 
     // ---- S0: r = b - A x, b.b and r.r partials, z = W^-1 r; level 0's
     // interpolation weights where level 0 is a grid level
     if (blockIdx.x == 0)
         for (int d = tid; d < P.ndom; d += blockDim.x) {
-            P.mgctl[d].active = (P.mgd[d].nlev > 0 && !P.dom[d].frozen) ? 1 : 0;
+            P.mgctl[d].active = (mgd(d).nlev > 0 && !dom(d).frozen) ? 1 : 0;
             if (!P.mgctl[d].active) {
                 P.octrl[d].iter = 0;
                 P.octrl[d].rr = 0.0;
                 P.octrl[d].bb = 0.0;
             }
         }
-    chunks(0, [&](int k, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
-        double v[2] = {0.0, 0.0};
-        points0(ch, g, [&](int i, int j) {
+    chunks0([&](auto nq, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
+        constexpr int NQ = decltype(nq)::value;
+        double vr[NQ], vb[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            vr[q] = vb[q] = 0.0;
+            if (tid + q * MG_THREADS >= ch.count) continue;
+            const int pt = ch.first + tid + q * MG_THREADS, i = pt % g.m[0], j = pt / g.m[0];
             const Lvl f = level(g, 0);
             const long long c = f.at(i, j);
             const OlfCoef cf = olf_coef(P, D, c, ctot);
@@ -923,15 +1034,12 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
             P.mg_w0[c] = w0;
             P.olf_r[c] = r;
             P.olf_z[c] = w0 * r;
-            v[0] += r * r;
-            v[1] += b * b;
+            vr[q] = r * r;
+            vb[q] = b * b;
             if (g.lc >= 1) weight_point(P, D, ctot, g, 0, i, j);
-        });
-        olf_block_sum<2>(v);
-        if (tid == 0) {
-            pslot(MP_RR, k) = v[0];
-            pslot(MP_BB, k) = v[1];
         }
+        group_sums(MP_RR, vr, ch, g);
+        group_sums(MP_BB, vb, ch, g);
     });
     if (!sync()) return;
     // ---- set-up of the grid levels: A_l and the restriction into level l,
@@ -956,9 +1064,9 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
     }
     // ---- set-up of every domain's block levels
     for (int d = blockIdx.x; d < P.ndom; d += gridDim.x) {
-        const MgDom &g = P.mgd[d];
+        const MgDom &g = mgd(d);
         if (g.nlev > 0) {
-            block_setup(P, P.dom[d], ctot, g, s_mg);
+            block_setup(P, dom(d), ctot, g, s_mg);
             if (tid == 0) s_resident = d;
         }
     }
@@ -973,9 +1081,9 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
         if (blockIdx.x == 0 && tid == 0) P.gctrl->olf_live[(it + 2) % 3] = 0;
         for (int d = blockIdx.x; d < P.ndom; d += gridDim.x) {
             if (!active(d)) continue;  // only this block writes the flag of d
-            const DomSums sm = decision_sums(P, P.mgd[d], it);
+            const DomSums sm = decision_sums(P, mgd(d), it);
             if (tid == 0) {
-                if (mg_stop(P.dom[d], it, sm.rr, sm.bb, sm.pq, sm.rz)) {
+                if (mg_stop(dom(d), it, sm.rr, sm.bb, sm.pq, sm.rz)) {
                     P.mgctl[d].active = 0;
                     P.octrl[d].iter = it;
                     P.octrl[d].rr = sm.rr;
@@ -993,8 +1101,8 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
             cache_dom = d;
             cache_live = active(d);
             if (cache_live) {
-                const DomSums sm = decision_sums(P, P.mgd[d], it);
-                cache_live = !mg_stop(P.dom[d], it, sm.rr, sm.bb, sm.pq, sm.rz);
+                const DomSums sm = decision_sums(P, mgd(d), it);
+                cache_live = !mg_stop(dom(d), it, sm.rr, sm.bb, sm.pq, sm.rz);
             }
         }
         return cache_live;
@@ -1023,9 +1131,9 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
             int cd = -1;
             bool cl = false;
             for (int d = blockIdx.x; d < P.ndom; d += gridDim.x) {
-                const MgDom &g = P.mgd[d];
+                const MgDom &g = mgd(d);
                 const bool go = Lg == 0 ? live_after(d, it, cd, cl) : active(d);
-                if (go && g.nlev > 0) block_vcycle(P, P.dom[d], ctot, g, d, s_mg, s_resident);
+                if (go && g.nlev > 0) block_vcycle(P, dom(d), ctot, g, d, s_mg, s_resident);
             }
         }
         if (!sync()) return;
@@ -1040,38 +1148,38 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
             if (!sync()) return;
         }
         // ---- level 0: z (the preconditioned residual, in olf_w) and r.z
-        chunks(0, [&](int k, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
+        chunks0([&](auto nq, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
             if (!active(ch.dom)) return;
             // every point's value first, then the stores (as in X and Y)
-            constexpr int NQ = MG_CHUNK0 / OLF_THREADS;
+            constexpr int NQ = decltype(nq)::value;
             const Lvl f = level(g, 0);
             long long cq[NQ];
             double tq[NQ], rq[NQ];
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
-                const int o = tid + q * OLF_THREADS;
+                const int o = tid + q * MG_THREADS;
                 const int pt = ch.first + (o < ch.count ? o : 0);
                 const int i = pt % f.m, j = pt / f.m;
                 cq[q] = f.at(i, j);
                 tq[q] = g.lc > 0 ? smooth_up_value<true>(P, D, ctot, g, 0, i, j) : __ldcg(P.olf_w + cq[q]);
                 rq[q] = __ldcg(P.olf_r + cq[q]);
             }
-            double v[1] = {0.0};
+            double v[NQ];
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
-                if (tid + q * OLF_THREADS >= ch.count) continue;
+                v[q] = 0.0;
+                if (tid + q * MG_THREADS >= ch.count) continue;
                 if (g.lc > 0) P.olf_w[cq[q]] = tq[q];
-                v[0] += rq[q] * tq[q];
+                v[q] = rq[q] * tq[q];
             }
-            olf_block_sum<1>(v);
-            if (tid == 0) pslot(MP_RZ + (it & 1), k) = v[0];
+            group_sums(MP_RZ + (it & 1), v, ch, g);
         });
         if (!sync()) return;
         // ---- X: p = z + beta p, q = A z + beta q, p.q
         {
             int cd = -1;
             double beta = 0.0;
-            chunks(0, [&](int k, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
+            chunks0([&](auto nq, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
                 if (!active(ch.dom)) return;
                 if (ch.dom != cd) {
                     cd = ch.dom;
@@ -1082,13 +1190,13 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
                 }
                 // every point's loads first, then the stores (the compiler may
                 // not move a point's loads across an earlier point's stores)
-                constexpr int NQ = MG_CHUNK0 / OLF_THREADS;
+                constexpr int NQ = decltype(nq)::value;
                 const Lvl f = level(g, 0);
                 long long cq[NQ];
                 double zq[NQ], azq[NQ], pq0[NQ], sq0[NQ];
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) {
-                    const int o = tid + q * OLF_THREADS;
+                    const int o = tid + q * MG_THREADS;
                     const int pt = ch.first + (o < ch.count ? o : 0);
                     cq[q] = f.at(pt % f.m, pt / f.m);
                     const OlfCoef cf = olf_coef(P, D, cq[q], ctot);
@@ -1097,18 +1205,18 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
                     pq0[q] = it == 0 ? 0.0 : __ldcg(P.olf_p + cq[q]);
                     sq0[q] = it == 0 ? 0.0 : __ldcg(P.olf_s + cq[q]);
                 }
-                double pq[1] = {0.0};
+                double pq[NQ];
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) {
-                    if (tid + q * OLF_THREADS >= ch.count) continue;
+                    pq[q] = 0.0;
+                    if (tid + q * MG_THREADS >= ch.count) continue;
                     const double p = it == 0 ? zq[q] : zq[q] + beta * pq0[q];
                     const double qv = it == 0 ? azq[q] : azq[q] + beta * sq0[q];
                     P.olf_p[cq[q]] = p;
                     P.olf_s[cq[q]] = qv;
-                    pq[0] += p * qv;
+                    pq[q] = p * qv;
                 }
-                olf_block_sum<1>(pq);
-                if (tid == 0) pslot(MP_PQ, k) = pq[0];
+                group_sums(MP_PQ, pq, ch, g);
             });
         }
         if (!sync()) return;
@@ -1116,7 +1224,7 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
         {
             int cd = -1;
             double alpha = 0.0;
-            chunks(0, [&](int k, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
+            chunks0([&](auto nq, const MgChunk &ch, const MgDom &g, const DomainDesc &D) {
                 if (!active(ch.dom)) return;
                 if (ch.dom != cd) {
                     cd = ch.dom;
@@ -1125,13 +1233,13 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
                     chunk_sums<2>(P, g, slots, v);
                     alpha = (v[1] > 0.0 && v[0] > 0.0 && v[1] < 1e300) ? v[0] / v[1] : 0.0;
                 }
-                constexpr int NQ = MG_CHUNK0 / OLF_THREADS;
+                constexpr int NQ = decltype(nq)::value;
                 const Lvl f = level(g, 0);
                 long long cq[NQ];
                 double hq[NQ], pq[NQ], rq[NQ], sq[NQ], wq[NQ];
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) {
-                    const int o = tid + q * OLF_THREADS;
+                    const int o = tid + q * MG_THREADS;
                     const int pt = ch.first + (o < ch.count ? o : 0);
                     cq[q] = f.at(pt % f.m, pt / f.m);
                     hq[q] = __ldcg(P.H + cq[q]);
@@ -1140,18 +1248,18 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
                     sq[q] = __ldcg(P.olf_s + cq[q]);
                     wq[q] = __ldcg(P.mg_w0 + cq[q]);
                 }
-                double rr[1] = {0.0};
+                double rr[NQ];
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) {
-                    if (tid + q * OLF_THREADS >= ch.count) continue;
+                    rr[q] = 0.0;
+                    if (tid + q * MG_THREADS >= ch.count) continue;
                     P.H[cq[q]] = hq[q] + alpha * pq[q];
                     const double r = rq[q] - alpha * sq[q];
                     P.olf_r[cq[q]] = r;
                     P.olf_z[cq[q]] = wq[q] * r;
-                    rr[0] += r * r;
+                    rr[q] = r * r;
                 }
-                olf_block_sum<1>(rr);
-                if (tid == 0) pslot(MP_RR, k) = rr[0];
+                group_sums(MP_RR, rr, ch, g);
             });
         }
         if (!sync()) return;
@@ -1160,7 +1268,7 @@ __global__ void __launch_bounds__(OLF_THREADS, 2) k_olf_mgcg(DevPtrs P, long lon
 
 // ------------------------------------------------------------------- host
 bool mg_plan(const std::vector<DomainDesc> &doms, std::vector<MgDom> &mgd, std::vector<MgChunk> &chunks,
-             int (&lchunk)[MG_MAXLEV + 2], int &lg, long long &nc, long long &npw, long long &ndinv) {
+             int (&lchunk)[MG_MAXLEV + 2], int &lg, long long &nc, long long &npw, long long &ndinv, int blocks, int &size0) {
     const int nd = (int)doms.size();
     mgd.assign(nd, MgDom{});
     nc = npw = ndinv = 0;
@@ -1202,6 +1310,14 @@ bool mg_plan(const std::vector<DomainDesc> &doms, std::vector<MgDom> &mgd, std::
         }
         lg = std::max(lg, g.lc);
     }
+    // level-0 chunks: as few groups each as give every block of an SM at most one
+    // (a group more is a point more per thread in every phase of the CG: 512x512
+    // with 1 / 2 / 4 groups 2.85 / 2.50 / 2.29 ms, 61x47 0.60 / 0.67 / 0.83)
+    long long groups = 0;
+    for (int d = 0; d < nd; ++d)
+        if (mgd[d].nlev > 0) groups += (mgd[d].m[0] * mgd[d].n[0] + MG_THREADS - 1) / MG_THREADS;
+    size0 = 1;
+    while (size0 < MG_CHUNK0 && groups > (long long)size0 * blocks) size0 *= 2;
     // chunk lists: level 0 for every domain with an interior (the CG's
     // vectors), level l >= 1 for the domains whose grid phases write it
     chunks.clear();
@@ -1213,7 +1329,7 @@ bool mg_plan(const std::vector<DomainDesc> &doms, std::vector<MgDom> &mgd, std::
             if (g.nlev == 0 || (l > 0 && l > g.lc)) continue;
             const int tot = g.m[l] * g.n[l];
             if (l == 0) g.c0_first = (int)chunks.size();
-            const int csize = l == 0 ? MG_CHUNK0 : OLF_THREADS;
+            const int csize = l == 0 ? size0 * MG_THREADS : MG_THREADS;
             for (int f = 0; f < tot; f += csize) chunks.push_back(MgChunk{d, l, f, std::min(csize, tot - f)});
             if (l == 0) g.c0_count = (int)chunks.size() - g.c0_first;
         }
@@ -1229,7 +1345,7 @@ cudaError_t configure_mg(LaunchCfg &L, int device) {
     e = cudaFuncSetAttribute((const void *)k_olf_mgcg, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM_BYTES);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_olf_mgcg, OLF_THREADS, MG_SMEM_BYTES);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_olf_mgcg, MG_THREADS, MG_SMEM_BYTES);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     L.mg_blocks = per_sm * prop.multiProcessorCount;
@@ -1243,6 +1359,6 @@ cudaError_t launch_overland_mg(const DevPtrs &P, const LaunchCfg &L, long long c
     int need = P.ndom;
     for (int l = 0; l <= P.mg_lg; ++l) need = std::max(need, P.mg_lchunk[l + 1] - P.mg_lchunk[l]);
     const int grid = std::max(1, std::min(L.mg_blocks, need));
-    return cudaLaunchCooperativeKernel((const void *)k_olf_mgcg, dim3(grid), dim3(OLF_THREADS), kargs, MG_SMEM_BYTES,
+    return cudaLaunchCooperativeKernel((const void *)k_olf_mgcg, dim3(grid), dim3(MG_THREADS), kargs, MG_SMEM_BYTES,
                                        s);
 }
