@@ -1792,11 +1792,13 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom) {
     L.krylov_per_sm = per_sm;
     L.step_per_sm = step_sm < per_sm ? step_sm : per_sm;
     if (L.step_per_sm < 1) return cudaErrorInvalidConfiguration;
-    // one launch per subsurface step by default, where the fused kernel keeps
-    // the Krylov kernel's occupancy; the pipelined solve's block has too few warps
-    // for the assembly (32x32x20 FP64 two steps 6.1 fused, 5.75 ms separate,
-    // 512x512x40 FP64 92 / 84.7)
+    // one launch per subsurface step by default, where the fused kernel keeps the
+    // Krylov kernel's occupancy, but not with the pipelined solve, whose block has too
+    // few warps for the assembly (32x32x20 FP64 two steps 6.1 fused, 5.75 ms separate,
+    // 512x512x40 FP64 92 / 84.7), nor for several domains, whose uneven tiles the fused
+    // kernel's blocks share less well (256 domains 250 / 235; one domain of
+    // 1024x1024x50 320 / 327, of 512x512x40 59.1 / 58.8)
     L.pipe = use_pipe(L, ntiles, ndom);
-    L.fused_step = !L.pipe && L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
+    L.fused_step = !L.pipe && ndom == 1 && L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
     return cudaSuccess;
 }

@@ -322,8 +322,8 @@ typedef struct {
     double overland_ms;
     /* 1: each subsurface step is one persistent launch (prologue, every Picard
      * iteration's assembly, solve and check, epilogue) -- the default where
-     * that kernel runs as many blocks per SM as the Krylov kernel and the solve is
-     * not the pipeline; 0: a launch
+     * that kernel runs as many blocks per SM as the Krylov kernel and the handle
+     * has one domain and not the pipelined solve; 0: a launch
      * per kernel (per-kernel timing then names every phase).  Results are the
      * same bit for bit. */
     int32_t fused_step;
