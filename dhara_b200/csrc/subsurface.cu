@@ -4,8 +4,8 @@
 // Kernel map (reference -> here):
 //   EstimateFluxes + IdentifyTopBoundary (src/global.cu:172-257)  -> k_prologue
 //   vanGenuchten + SetUpLinearSystemsSubsurface (subsurface.cu:381-429)
-//     + ModifiedPicardUpdate (450-461)                             -> k_assemble
-//   CUSP BiCGSTAB on the DIA matrix (subsurface.cu:750-751)        -> k_krylov
+//     + ModifiedPicardUpdate (450-461)              -> k_assemble(_planes)
+//   CUSP BiCGSTAB on the DIA matrix (subsurface.cu:750-751)        -> k_krylov(_pipe)
 //   GetIterationDifference + max_element (432-446, 762-789)        -> k_picard_check
 //   vanGenuchten + SubsurfaceEstimateInfiltrationPonding (465-491)
 //     + WaterFluxEstimate + reductions (494-629, 809-826)
