@@ -836,9 +836,13 @@ __device__ __forceinline__ void finalize_C(const DevPtrs &P, int dom, KrylovCtrl
 }
 
 // The sums of a domain's partials (a warp; lane 0 gets them).  A phase's are not
-// overwritten in the next one, where a slow block may still be reading them.
+// overwritten in the next one, where a slow block may still be reading them; nor
+// by the Picard check (row 0), which follows a solve's last phase R in k_step_pipe
+// with no barrier between them.
+enum { PART_ROW0 = 4 };
+static_assert(PART_ROW0 + 8 <= NPART, "four rows each for even and odd phases");
 __device__ __forceinline__ double *part_at(const DevPtrs &P, unsigned phase, int i, int t) {
-    return P.partials + ((size_t)(4 * (phase & 1u)) + i) * P.ntiles + t;
+    return P.partials + ((size_t)(PART_ROW0 + 4 * (phase & 1u)) + i) * P.ntiles + t;
 }
 __device__ __forceinline__ void sum_parts(const DevPtrs &P, unsigned phase, int begin, int parts, double (&v)[4]) {
     const int lane = threadIdx.x & 31;

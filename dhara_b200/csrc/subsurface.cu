@@ -1314,6 +1314,7 @@ __device__ __forceinline__ void picard_check_tile(const DevPtrs &P, int tile) {
     }
     if (nonfinite) atomicOr(&P.diag[td.dom].nonfinite, 1);
     double v[1] = {mx};
+    static_assert(sizeof(v) / sizeof(v[0]) <= pipe::PART_ROW0, "the pipelined solve's last sums may still be being read");
     if (domain_reduce<1, true, G>(P, tile, td.dom, 1, v) && tile_thread<G>() == 0) {
         PicardCtrl &c = P.pctrl[td.dom];
         DevDiag &dg = P.diag[td.dom];
