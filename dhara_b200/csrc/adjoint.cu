@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_adj_matrix(DevPtrs P, AdjPtrs 
     const int tile = blockIdx.x;
     const TileDesc td = P.tiles[tile];
     const DomainDesc &D = P.dom[td.dom];
-    if (threadIdx.x == 0 && tile == 0) P.gctrl->kry_bar = 0;
+    if (threadIdx.x == 0 && tile == 0) solve_begin(P);
     if (threadIdx.x == 0 && tile == D.tile_begin) {
         KrylovCtrl &kc = P.kctrl[td.dom];
         kc.active = 1;

@@ -1721,7 +1721,7 @@ int dhara_adjoint(dhara_handle *h, const dhara_adjoint_desc *desc, double *loss,
             const int Mi = iters[sl] < 1 ? 1 : (iters[sl] > M ? M : iters[sl]);
             LAUNCH(KT_ADJOINT, launch_adj_epilogue(P, A, sl, Mi, s));
             for (int m = Mi - 1; m >= 0; --m) {
-                CK(cudaMemsetAsync(&P.gctrl->n_active, 0, 2 * sizeof(int), s));
+                CK(cudaMemsetAsync(&P.gctrl->n_active, 0, sizeof(int), s));
                 LAUNCH(KT_ADJOINT, launch_adj_matrix(P, A, sl, m, m == Mi - 1, h->mixed, s));
                 LAUNCH(KT_KRYLOV, launch_krylov(P, h->L, s));
                 LAUNCH(KT_ADJOINT, launch_adj_picard(P, A, sl, m, s));

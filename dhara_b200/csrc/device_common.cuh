@@ -112,6 +112,23 @@ __device__ __forceinline__ bool counter_sync(unsigned int *count, unsigned int t
     return counter_sync(count, target, gb, [] {});
 }
 
+// ------------------------------------------------------------ live domains
+// The domains whose inner solve goes on after a phase of the 3D solve (R, an inner
+// sweep, U: each ends with a grid barrier), counted during the phase in slot
+// phase % 3 and read after its barrier.  A block without tiles of the last live
+// domains may read late, while the others are in the next phase, so that one must
+// not change the slot (one counter for all phases let such a block leave the loop a
+// barrier early); it is cleared in the phase after, when every block has read it.
+__device__ __forceinline__ int *live_slot(const DevPtrs &P, unsigned int phase) { return &P.gctrl->kry_live[phase % 3u]; }
+__device__ __forceinline__ void live_begin(const DevPtrs &P, unsigned int phase) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *live_slot(P, phase + 1) = 0;
+}
+// Before a solve (one thread of the kernel or phase ahead of it).
+__device__ __forceinline__ void solve_begin(const DevPtrs &P) {
+    P.gctrl->kry_bar = 0;
+    for (int q = 0; q < 3; ++q) P.gctrl->kry_live[q] = 0;
+}
+
 // ------------------------------------------------------------ tile groups
 // Tiles are worked on by groups of TILE_THREADS threads: the whole block (G = 1)
 // in most kernels, G groups of a larger block in k_step_pipe.  These meet at a

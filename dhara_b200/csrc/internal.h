@@ -247,12 +247,12 @@ struct GridBarrier {
 // Global counters for the persistent kernels.
 struct GlobalCtrl {
     int n_active;        // domains with an active outer solve
-    int n_inner_active;  // domains with an active inner solve
     int n_olf_active;
     unsigned int olf_bar;  // arrivals at the resident overland solve's barrier
     int olf_live[4];     // domains still iterating, rotating over three phases
     int n_picard;        // domains whose Picard iteration is not done this step (k_step)
     unsigned int kry_bar;  // arrivals at the pipelined solve's barrier (zeroed by the assembly before it)
+    int kry_live[3];       // domains whose inner solve goes on, rotating over three phases (zeroed there too)
 };
 
 // Number of double partial sums per tile kept for reductions.

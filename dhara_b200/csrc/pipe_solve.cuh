@@ -776,8 +776,10 @@ __device__ __forceinline__ void columns_done(Pipe &pp, int nz) {
 
 // The decisions after a phase R and after an inner sweep, on a domain's control
 // record from its sums.  `report`: also into the domain's diagnostics and the
-// counts of live domains.
-__device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, KrylovCtrl &c, bool report, const double (&v)[4]) {
+// count of active domains.  live: the phase's count of live domains (null with
+// one domain, whose record tells).
+__device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, KrylovCtrl &c, bool report, int *live,
+                                           const double (&v)[4]) {
     const DomainDesc &D = P.dom[dom];
     const double rr64 = v[0], bb = v[1];
     c.bb = bb;
@@ -797,7 +799,7 @@ __device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, KrylovCtrl
         }
     } else {
         c.inner_active = 1;
-        if (report) atomicAdd(&P.gctrl->n_inner_active, 1);
+        if (live) atomicAdd(live, 1);
         c.inner_iter = 0;
         c.first_inner = 1;
         c.rz = v[2];
@@ -815,7 +817,7 @@ __device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, KrylovCtrl
     }
 }
 
-__device__ __forceinline__ void finalize_C(const DevPtrs &P, int dom, KrylovCtrl &c, bool report, const double (&v)[4]) {
+__device__ __forceinline__ void finalize_C(const DevPtrs &P, int dom, KrylovCtrl &c, int *live, const double (&v)[4]) {
     const DomainDesc &D = P.dom[dom];
     const double sigma = v[0], mu = v[1], nu = v[2], rho = v[3];
     const double alpha = rho / sigma;
@@ -829,10 +831,10 @@ __device__ __forceinline__ void finalize_C(const DevPtrs &P, int dom, KrylovCtrl
     c.first_inner = 0;
     c.inner_iter += 1;
     c.total_iter += 1;
-    if (bad || rho_next <= c.inner_target2 || c.inner_iter >= D.inner_maxiter || c.total_iter >= D.krylov_maxiter) {
+    if (bad || rho_next <= c.inner_target2 || c.inner_iter >= D.inner_maxiter || c.total_iter >= D.krylov_maxiter)
         c.inner_active = 0;
-        if (report) atomicSub(&P.gctrl->n_inner_active, 1);
-    }
+    else if (live)
+        atomicAdd(live, 1);
 }
 
 // The sums of a domain's partials (a warp; lane 0 gets them).  A phase's are not
@@ -901,8 +903,8 @@ __device__ __forceinline__ void block_reduce(const DevPtrs &P, Pipe &pp, PipeSha
     sum_parts(P, phase, td.begin, parts, v);
     if (lane != 0) return;
     P.arrive[td.dom * 4] = 0u;
-    if (RESIDUAL) finalize_R(P, td.dom, P.kctrl[td.dom], true, v);
-    else finalize_C(P, td.dom, P.kctrl[td.dom], true, v);
+    if (RESIDUAL) finalize_R(P, td.dom, P.kctrl[td.dom], true, live_slot(P, phase), v);
+    else finalize_C(P, td.dom, P.kctrl[td.dom], live_slot(P, phase), v);
 }
 
 // One domain: every block sums the partials after the grid barrier and keeps the
@@ -915,8 +917,8 @@ __device__ __forceinline__ void decide(const DevPtrs &P, SolveBlock &b) {
         sum_parts(P, b.phase - 1, 0, P.ntiles < grid ? P.ntiles : grid, v);
         if (threadIdx.x == 0) {
             const bool report = blockIdx.x == 0;
-            if (RESIDUAL) finalize_R(P, 0, b.sh->ctl, report, v);
-            else finalize_C(P, 0, b.sh->ctl, report, v);
+            if (RESIDUAL) finalize_R(P, 0, b.sh->ctl, report, nullptr, v);
+            else finalize_C(P, 0, b.sh->ctl, nullptr, v);
             if (report) P.kctrl[0] = b.sh->ctl;
         }
     }
@@ -932,6 +934,7 @@ template <typename T, int TXC, bool RESIDUAL>
 __device__ __forceinline__ void run_sweep(const DevPtrs &P, SolveBlock &b, int role) {
     Pipe &pp = RESIDUAL ? b.r : b.c;
     SweepCtl c{-1, 0, 0, false, false, 0.0, 0.0};
+    live_begin(P, b.phase);
     // fn(tile, its record, how many tiles of its domain the block had before,
     // whether it is the block's last one) for every tile of a live domain
     auto each_tile = [&](auto fn) {
@@ -1137,12 +1140,13 @@ __device__ __forceinline__ bool solve(const DevPtrs &P, SolveBlock &b) {
         if (one) decide<true>(P, b);
         if (one ? b.sh->ctl.active == 0 : ldcg(&P.gctrl->n_active) == 0) break;
         // ---- inner PCG: one sweep and one grid barrier per iteration
-        while (one ? b.sh->ctl.inner_active != 0 : ldcg(&P.gctrl->n_inner_active) > 0) {
+        while (one ? b.sh->ctl.inner_active != 0 : ldcg(live_slot(P, b.phase - 1)) > 0) {
             run_sweep<T, TXC, false>(P, b, role);
             if (!solve_sync(P, b)) return fail();
             if (one) decide<false>(P, b);
         }
         // ---- U
+        live_begin(P, b.phase);
         update_x<T>(P, b);
         if (!solve_sync(P, b)) return fail();
     }

@@ -134,7 +134,6 @@ __device__ __forceinline__ void prologue_tile(const DevPtrs &P, int tile) {
     if (tile_thread<G>() == 0) {
         if (tile == 0) {
             P.gctrl->n_active = 0;
-            P.gctrl->n_inner_active = 0;
             P.gctrl->n_olf_active = 0;
             P.gctrl->n_picard = P.ndom - P.n_frozen;
         }
@@ -205,7 +204,7 @@ __global__ void k_prologue(DevPtrs P) {
 __device__ __forceinline__ bool assemble_begin(const DevPtrs &P, int tile, bool first_thread) {
     const TileDesc td = P.tiles[tile];
     const int done = P.pctrl[td.dom].done;
-    if (first_thread && tile == 0) P.gctrl->kry_bar = 0;
+    if (first_thread && tile == 0) solve_begin(P);
     if (first_thread && tile == P.dom[td.dom].tile_begin) {
         KrylovCtrl &kc = P.kctrl[td.dom];
         kc.active = done ? 0 : 1;
@@ -1039,7 +1038,7 @@ __device__ __forceinline__ void phase_C(const DevPtrs &P, int tile, int tile_nex
     if (cr.valid) back_sweep<T, DSMEM>(cr, s_d, fc, t_out);
 }
 
-__device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, const double (&v)[3]) {
+__device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, int *live, const double (&v)[3]) {
     KrylovCtrl &c = P.kctrl[dom];
     const DomainDesc &D = P.dom[dom];
     const double rr64 = v[0], bb = v[1];
@@ -1058,7 +1057,7 @@ __device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, const doub
         dg.krylov_relres_last = bb > 0 ? sqrt(rr64 / bb) : sqrt(rr64);
     } else {
         c.inner_active = 1;
-        atomicAdd(&P.gctrl->n_inner_active, 1);
+        atomicAdd(live, 1);
         c.inner_iter = 0;
         c.first_inner = 1;
         c.rz = v[2];
@@ -1074,11 +1073,6 @@ __device__ __forceinline__ void finalize_R(const DevPtrs &P, int dom, const doub
         // the M^-1-norm standing in for the 2-norm); R checks the true residual
         c.inner_target2 = v[2] * fmax(D.inner_tol * D.inner_tol, 0.25 * tol2 * bb / rr64);
     }
-}
-
-__device__ __forceinline__ void stop_inner(const DevPtrs &P, KrylovCtrl &c) {
-    c.inner_active = 0;
-    atomicSub(&P.gctrl->n_inner_active, 1);
 }
 
 // Shared memory of the persistent 3D solve: [d' of the column solves (float
@@ -1130,9 +1124,11 @@ __device__ __forceinline__ bool krylov_solve(const DevPtrs &P, const SolveSmem<T
         const DomainDesc &D = P.dom[dom];
         return StencilW<T>{(T)(1.0 / (D.dx * D.dx)), (T)(1.0 / (D.dy * D.dy)), (T)(1.0 / (D.dz * D.dz))};
     };
+    unsigned int phase = 0;  // grid barriers passed
     for (;;) {
         // ---- R: outer residual
         {
+            live_begin(P, phase);
             bool pre = false;
             for (int t = next_outer(blockIdx.x); t < P.ntiles;) {
                 const int tn = next_outer(t + gridDim.x);
@@ -1146,11 +1142,12 @@ __device__ __forceinline__ bool krylov_solve(const DevPtrs &P, const SolveSmem<T
                 else
                     phase_R<T, DSMEM, 16>(P, t, tn, pre, cr, weights(dom), s_d, stage_raw, sb, v);
                 pre = tn < P.ntiles;
-                if (domain_reduce<3>(P, t, dom, 0, v) && threadIdx.x == 0) finalize_R(P, dom, v);
+                if (domain_reduce<3>(P, t, dom, 0, v) && threadIdx.x == 0) finalize_R(P, dom, live_slot(P, phase), v);
                 t = tn;
             }
         }
         if (!grid_sync(P.barrier)) return fail();
+        phase += 1;
         if (ldcg(&P.gctrl->n_active) == 0) break;
         // ---- inner PCG: one sweep and one grid barrier per iteration
         // A domain's control record (inner_active, parity, first_inner, alpha,
@@ -1182,7 +1179,8 @@ __device__ __forceinline__ bool krylov_solve(const DevPtrs &P, const SolveSmem<T
             }
             return t;
         };
-        while (ldcg(&P.gctrl->n_inner_active) > 0) {
+        while (ldcg(live_slot(P, phase - 1)) > 0) {
+            live_begin(P, phase);
             bool pre = false;
             Ctl cc{-1, 0, 0, false, false, 0.0, 0.0}, cn{-1, 0, 0, false, false, 0.0, 0.0};
             for (int t = next_live(cc, blockIdx.x); t < P.ntiles;) {
@@ -1222,13 +1220,17 @@ __device__ __forceinline__ bool krylov_solve(const DevPtrs &P, const SolveSmem<T
                     c.total_iter += 1;
                     if (bad || rho_next <= c.inner_target2 || c.inner_iter >= D.inner_maxiter ||
                         c.total_iter >= D.krylov_maxiter)
-                        stop_inner(P, c);
+                        c.inner_active = 0;
+                    else
+                        atomicAdd(live_slot(P, phase), 1);
                 }
                 t = tn;
             }
             if (!grid_sync(P.barrier)) return fail();
+            phase += 1;
         }
         // ---- U: x += d + alpha p (the last iteration's pending update)
+        live_begin(P, phase);
         for (int t = blockIdx.x; t < P.ntiles; t += gridDim.x) {
             const int dom = P.tiles[t].dom;
             const KrylovCtrl *kc = &P.kctrl[dom];
@@ -1246,6 +1248,7 @@ __device__ __forceinline__ bool krylov_solve(const DevPtrs &P, const SolveSmem<T
             }
         }
         if (!grid_sync(P.barrier)) return fail();
+        phase += 1;
     }
     return true;
 }
@@ -1270,7 +1273,6 @@ __device__ __forceinline__ void picard_check_tile(const DevPtrs &P, int tile) {
     const TileDesc td = P.tiles[tile];
     if (tile == 0 && tile_thread<G>() == 0) {
         P.gctrl->n_active = 0;
-        P.gctrl->n_inner_active = 0;
     }
     const PicardCtrl &pc = P.pctrl[td.dom];
     if (pc.done) return;
