@@ -1100,9 +1100,12 @@ __device__ __forceinline__ SolveBlock solve_block(const DevPtrs &P, unsigned cha
 
 // Grid barrier of the solve: a counter (zeroed by the assembly before it) that
 // every block adds to once per phase.  What the phase wrote is read by the TMA
-// in the next one, so both sides order it for the async proxy.
+// in the next one, so both sides order it for the async proxy.  So is what it
+// wrote to shared memory: the two kinds of sweep may have another number of
+// column buffers (FP64 columns of 26 to 35 layers, mixed ones of 48 and 49), and
+// one's second buffer is then where the other's TMA writes its first stages.
 __device__ __forceinline__ bool solve_sync(const DevPtrs &P, SolveBlock &b) {
-    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+    asm volatile("fence.proxy.async;\n" ::: "memory");
     b.target += gridDim.x;
     b.phase += 1;
     const bool ok = counter_sync(&P.gctrl->kry_bar, b.target, P.barrier);
