@@ -1135,6 +1135,9 @@ __device__ __forceinline__ bool solve(const DevPtrs &P, SolveBlock &b) {
     if (one) {
         if (threadIdx.x == 0) b.sh->ctl = P.kctrl[0];
         __syncthreads();
+        // its Picard iteration has converged: no sweep would visit a tile, and there
+        // are no sums to decide on
+        if (b.sh->ctl.active == 0) return true;
     }
     for (;;) {
         // ---- R: outer residual
