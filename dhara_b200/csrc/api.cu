@@ -58,6 +58,7 @@ struct dhara_handle {
     size_t tiles_cap = 0;   // capacity of the device tile list and per-tile partials
     std::vector<OlfSeg> hsegs;
     long long Ntot = 0, Ctot = 0, WEtot = 0, SNtot = 0;
+    long long Nslab = 0;    // Ntot rounded up to 32: the arrays of one allocation start as aligned as its base
     DevPtrs P{};
     LaunchCfg L{};
     std::vector<void *> allocs;
@@ -427,6 +428,8 @@ int encode_map(CUtensorMap *m, const void *array, size_t elt, const DomainDesc &
     return DHARA_OK;
 }
 
+long long slab_cells(long long cells) { return (cells + 31) & ~31LL; }
+
 // The pipelined solve's maps: STAGE_PLANES planes of `arrays` arrays, `apart`
 // elements from one to the next, in one box.
 int encode_pipe_map(CUtensorMap *m, const void *array, size_t elt, const DomainDesc &D, bool halo, int arrays = 1,
@@ -453,7 +456,7 @@ int encode_pipe_map(CUtensorMap *m, const void *array, size_t elt, const DomainD
 int build_tensor_maps(dhara_handle *h) {
     const DevPtrs &P = h->P;
     const size_t sF = FACTOR_BYTES(h->mixed);
-    const long long N = h->Ntot;
+    const long long N = h->Nslab;
     const size_t sT = h->mixed ? 4 : 8;
     const int chi = h->mixed ? CHUNK_F32 : CHUNK_F64;
     std::vector<CUtensorMap> maps((size_t)h->ndom * NMAP);
@@ -723,7 +726,7 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
         if (p.nz > h->nz_max) h->nz_max = p.nz;
         if (p.picard_maxiter > h->maxiter_picard) h->maxiter_picard = p.picard_maxiter;
     }
-    h->Ntot = (h->Ntot + 31) & ~31LL;  // arrays of one allocation start as aligned as its base
+    h->Nslab = slab_cells(h->Ntot);
     // the inner sweeps index cells with 32-bit offsets
     if (h->Ntot >= (1LL << 31))
         return bail(fail(DHARA_ERR_UNSUPPORTED, "a handle holds at most 2^31 - 1 cells (with row padding); got %lld",
@@ -739,7 +742,7 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
     h->face_dirichlet.assign(ndomains, std::vector<bool>(5, false));
 
     DevPtrs &P = h->P;
-    const size_t N = (size_t)h->Ntot, C = (size_t)h->Ctot;
+    const size_t N = (size_t)h->Ntot, S = (size_t)h->Nslab, C = (size_t)h->Ctot;
     const size_t sT = h->mixed ? sizeof(float) : sizeof(double);
     int rc = 0;
     rc |= dalloc(h, &h->d_dom, ndomains);
@@ -751,21 +754,21 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
     // c', d where the factors have the inner precision, else D, d and the factors
     const size_t sF = FACTOR_BYTES(h->mixed);
     char *ztp = nullptr, *own = nullptr, *fac = nullptr;
-    rc |= dalloc(h, &ztp, 6 * N * sT);
-    rc |= dalloc(h, &own, (sF == sT ? 4 : 2) * N * sT);
-    if (sF != sT) rc |= dalloc(h, &fac, 2 * N * sF);
+    rc |= dalloc(h, &ztp, 6 * S * sT);
+    rc |= dalloc(h, &own, (sF == sT ? 4 : 2) * S * sT);
+    if (sF != sT) rc |= dalloc(h, &fac, 2 * S * sF);
     rc |= dalloc_void(h, &P.K, N * sT);
     if (rc) return bail(DHARA_ERR_NOMEM);
     P.z0 = ztp;
-    P.t0 = ztp + N * sT;
-    P.p0 = ztp + 2 * N * sT;
-    P.z1 = ztp + 3 * N * sT;
-    P.t1 = ztp + 4 * N * sT;
-    P.p1 = ztp + 5 * N * sT;
+    P.t0 = ztp + S * sT;
+    P.p0 = ztp + 2 * S * sT;
+    P.z1 = ztp + 3 * S * sT;
+    P.t1 = ztp + 4 * S * sT;
+    P.p1 = ztp + 5 * S * sT;
     P.D = own;
-    P.finv = fac ? fac : own + N * sT;
-    P.fc = fac ? fac + N * sF : own + 2 * N * sT;
-    P.d = own + (fac ? 1 : 3) * N * sT;
+    P.finv = fac ? fac : own + S * sT;
+    P.fc = fac ? fac + S * sF : own + 2 * S * sT;
+    P.d = own + (fac ? 1 : 3) * S * sT;
     if (h->mixed) {
         rc |= dalloc(h, &P.K64, N);
         rc |= dalloc(h, &P.D64, N);
@@ -1995,11 +1998,12 @@ struct CkptHeader {
 constexpr int32_t CKPT_VERSION = 2;
 constexpr int CKPT_DIM_INTS = 3;  // nx, ny, nz per domain, after the header
 
-size_t ckpt_bytes(const dhara_handle *h) {
+size_t ckpt_bytes(const dhara_handle *h, long long ntot) {
     return sizeof(CkptHeader) + (size_t)h->ndom * CKPT_DIM_INTS * sizeof(int32_t) +
-           ((size_t)2 * h->Ntot + (size_t)4 * h->Ctot) * sizeof(double) +
+           ((size_t)2 * ntot + (size_t)4 * h->Ctot) * sizeof(double) +
            (size_t)h->ndom * (sizeof(PicardCtrl) + sizeof(DevDiag) + 2 * sizeof(int64_t));
 }
+size_t ckpt_bytes(const dhara_handle *h) { return ckpt_bytes(h, h->Ntot); }
 
 // The device arrays of the checkpoint, in buffer order, with their lengths.
 void ckpt_arrays(const dhara_handle *h, double *(&arr)[6], size_t (&len)[6]) {
@@ -2073,13 +2077,14 @@ int dhara_restore(dhara_handle *h, const void *buf, int64_t bytes) {
     std::memcpy(&hd, q, sizeof(hd));
     if (std::memcmp(hd.magic, "DHARACK", 8) != 0 || hd.version != CKPT_VERSION)
         return fail(DHARA_ERR_INVALID, "not a checkpoint of this library version");
-    if (hd.ndom != h->ndom || hd.ntot != h->Ntot || hd.ctot != h->Ctot ||
+    // (some builds of this version wrote psi and theta rounded up to the slab)
+    if (hd.ndom != h->ndom || (hd.ntot != h->Ntot && hd.ntot != h->Nslab) || hd.ctot != h->Ctot ||
         hd.pctrl_bytes != (int32_t)sizeof(PicardCtrl) || hd.diag_bytes != (int32_t)sizeof(DevDiag))
         return fail(DHARA_ERR_INVALID, "checkpoint of %d domains / %lld cells does not match this handle "
                     "(%d / %lld)", hd.ndom, (long long)hd.ntot, h->ndom, (long long)h->Ntot);
-    if (bytes < (int64_t)ckpt_bytes(h))
+    if (bytes < (int64_t)ckpt_bytes(h, hd.ntot))
         return fail(DHARA_ERR_INVALID, "checkpoint buffer of %lld bytes is smaller than %lld", (long long)bytes,
-                    (long long)ckpt_bytes(h));
+                    (long long)ckpt_bytes(h, hd.ntot));
     q += sizeof(hd);
     for (int d = 0; d < h->ndom; ++d) {
         int32_t dims[CKPT_DIM_INTS];
@@ -2097,7 +2102,7 @@ int dhara_restore(dhara_handle *h, const void *buf, int64_t bytes) {
     const DevPtrs &P = h->P;
     for (int i = 0; i < 6; ++i) {
         CK(cudaMemcpyAsync(arr[i], q, len[i] * sizeof(double), cudaMemcpyHostToDevice, s));
-        q += len[i] * sizeof(double);
+        q += (i < 2 ? (size_t)hd.ntot : len[i]) * sizeof(double);
     }
     // the Krylov warm start and the Picard iterate of a step's first
     // iteration are psi^n
