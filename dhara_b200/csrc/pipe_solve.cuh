@@ -131,29 +131,6 @@ struct StageR {
 // diagonal (the coupling is then left in the d array, which is free there).
 __host__ __device__ constexpr int col_bytes(int nz, int elt) { return TILE_THREADS * (elt + 8) * nz; }
 
-// a / b (b > 0, normal) for the sum z.M z.  FP32: the hardware's approximate
-// reciprocal (1 ulp) times a.  FP64: the approximate reciprocal refined by three
-// Newton-Raphson steps x <- x + x (1 - b x), each of which doubles the correct
-// digits, times a: within 1 ulp of a / b over 2^24 random pairs, without the
-// division's branches (solves of a pass, a / b / this: 53x37x21 FP64 1.35 / 1.18
-// ms, 512x512x40 FP64 73.4 / 71.2).
-template <typename T>
-__device__ __forceinline__ T quotient(T a, T b);
-template <>
-__device__ __forceinline__ float quotient(float a, float b) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-    return a * r;
-}
-template <>
-__device__ __forceinline__ double quotient(double a, double b) {
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
-#pragma unroll
-    for (int i = 0; i < 3; ++i) x = fma(x, fma(-b, x, 1.0), x);
-    return a * x;
-}
-
 // What the roles need to know of a tile.  A block's first TILE_TABLE tiles are
 // kept in shared memory for the whole solve: each sweep starts with a grid
 // barrier, after which the descriptors' lines are no longer in L1.
@@ -664,7 +641,7 @@ __device__ __forceinline__ void planes_C(const DevPtrs &P, const TileCtx &td, co
         constexpr T tiny = sizeof(T) == 4 ? T(1e-37) : T(1e-300);
         a[0] = fma2(pc, q, a[0]);
         a[1] = fma2(zc, q, a[1]);
-        a[2] = add2(a[2], mk2<T>(quotient(u.x, inv.x > tiny ? inv.x : tiny), quotient(u.y, inv.y > tiny ? inv.y : tiny)));
+        a[2] = add2(a[2], mk2<T>(quot(u.x, inv.x > tiny ? inv.x : tiny), quot(u.y, inv.y > tiny ? inv.y : tiny)));
         const unsigned g = r.g + (unsigned)(k - unit_plane()) * td.sxy;
         put2<T>(z_out + g, zc);
         put2<T>(p_out + g, pc);

@@ -45,22 +45,6 @@ struct Fac<double> {
 };
 #endif
 
-template <typename T>
-__device__ __forceinline__ T recip(T x);
-template <>
-__device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
-template <>
-__device__ __forceinline__ double recip(double x) { return 1.0 / x; }
-
-// a / b where the quotient only feeds a sum of positive terms (z.M z): the
-// hardware reciprocal's approximation (about 2 ulp) in FP32
-template <typename T>
-__device__ __forceinline__ T quot(T a, T b);
-template <>
-__device__ __forceinline__ float quot(float a, float b) { return __fdividef(a, b); }
-template <>
-__device__ __forceinline__ double quot(double a, double b) { return a / b; }
-
 #include "pipe_solve.cuh"
 
 // The closure of the assembled system: the reference's FP64 expressions in
