@@ -87,6 +87,13 @@ __device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
 __device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ double2 sub2(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// sum + a / b
+__device__ __forceinline__ float2 add_quot2(float2 sum, float2 a, float2 b) {
+    return add2(sum, make_float2(quot(a.x, b.x), quot(a.y, b.y)));
+}
+__device__ __forceinline__ double2 add_quot2(double2 sum, double2 a, double2 b) {
+    return make_double2(add_quot(sum.x, a.x, b.x), add_quot(sum.y, a.y, b.y));
+}
 template <typename T, typename F>
 __device__ __forceinline__ P2<T> get2(const F *p) {
     const P2<F> v = *reinterpret_cast<const P2<F> *>(p);
@@ -641,7 +648,7 @@ __device__ __forceinline__ void planes_C(const DevPtrs &P, const TileCtx &td, co
         constexpr T tiny = sizeof(T) == 4 ? T(1e-37) : T(1e-300);
         a[0] = fma2(pc, q, a[0]);
         a[1] = fma2(zc, q, a[1]);
-        a[2] = add2(a[2], mk2<T>(quot(u.x, inv.x > tiny ? inv.x : tiny), quot(u.y, inv.y > tiny ? inv.y : tiny)));
+        a[2] = add_quot2(a[2], u, mk2<T>(inv.x > tiny ? inv.x : tiny, inv.y > tiny ? inv.y : tiny));
         const unsigned g = r.g + (unsigned)(k - unit_plane()) * td.sxy;
         put2<T>(z_out + g, zc);
         put2<T>(p_out + g, pc);
