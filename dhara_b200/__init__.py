@@ -134,6 +134,7 @@ class Solver:
         _check(lib().dhara_create(arr, len(plist), device, ct.byref(h)))
         self.h = h
         self.params = plist
+        self._krylov_solver = 0  # set_launch_config
 
     def close(self):
         if getattr(self, "h", None):
@@ -191,15 +192,19 @@ class Solver:
         return c.as_dict()
 
     def set_launch_config(self, krylov_blocks_per_sm, overland_resident, overland_blocks_per_sm, tile_shape=None,
-                          fused_step=None):
+                          fused_step=None, krylov_solver=None):
         """Sets the block schedule; tile_shape 0 (per domain), 1 (32 x 4) or 2
-        (16 x 8), fused_step 0/1; None keeps the current value."""
+        (16 x 8), fused_step 0/1, krylov_solver 0 (by the tiles per SM, as at
+        first), 1 (the pipeline) or 2 (blocks); None keeps the current value."""
         cur = self.launch_config()
         c = _abi.LaunchConfig()
         c.krylov_blocks_per_sm, c.overland_resident = krylov_blocks_per_sm, overland_resident
         c.overland_blocks_per_sm = overland_blocks_per_sm
         c.tile_shape = cur["tile_shape"] if tile_shape is None else tile_shape
         c.fused_step = cur["fused_step"] if fused_step is None else fused_step
+        if krylov_solver is not None:
+            self._krylov_solver = krylov_solver
+        c.krylov_solver = self._krylov_solver
         _check(lib().dhara_set_launch_config(self.h, ct.byref(c)))
 
     def enable_statistics(self, max_steps):

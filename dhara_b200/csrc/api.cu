@@ -374,6 +374,7 @@ int apply_tiles(dhara_handle *h) {
     CK(cudaMemcpyAsync((void *)h->P.tiles, h->htiles.data(), sizeof(TileDesc) * h->htiles.size(),
                        cudaMemcpyHostToDevice, h->stream));
     h->P.ntiles = (int)h->htiles.size();
+    choose_solver(h->L, h->P.ntiles, h->ndom);
     int rc = upload_dom_desc(h);
     if (!rc) rc = build_tensor_maps(h);
     if (h->graph_exec) {
@@ -1817,6 +1818,7 @@ void fill_config(const dhara_handle *h, dhara_launch_config *out) {
     out->overland_blocks_per_sm = h->L.olf_stream_per_sm;
     out->tile_shape = h->tile_mode;
     out->fused_step = h->L.fused_step;
+    out->krylov_solver = h->L.pipe ? 1 : 2;
 }
 
 }  // namespace
@@ -1844,6 +1846,8 @@ int dhara_set_launch_config(dhara_handle *h, const dhara_launch_config *cfg) {
         const int rc = apply_tiles(h);
         if (rc) return rc;
     }
+    h->L.krylov_solver = cfg->krylov_solver == 1 || cfg->krylov_solver == 2 ? cfg->krylov_solver : 0;
+    choose_solver(h->L, h->P.ntiles, h->ndom);
     h->L.krylov_per_sm = cfg->krylov_blocks_per_sm;
     h->L.fused_step = cfg->fused_step ? 1 : 0;
     h->L.olf_allow_resident = cfg->overland_resident ? 1 : 0;
@@ -1922,10 +1926,11 @@ int dhara_autotune(dhara_handle *h, int trial_steps, dhara_launch_config *chosen
         const int r2 = apply_tiles(h);
         if (!rc) rc = r2;
     }
-    // 3D Krylov: blocks per SM
+    // 3D Krylov: blocks per SM (the pipeline always runs one)
     int best_k = L.krylov_per_sm;
     double best_kms = 1e300;
-    for (int b = 1; b <= L.krylov_per_sm_max && !rc; ++b) {
+    if (L.pipe && !rc) rc = trial(KT_KRYLOV, &best_kms);
+    for (int b = 1; b <= L.krylov_per_sm_max && !rc && !L.pipe; ++b) {
         L.krylov_per_sm = b;
         double ms = 0;
         rc = trial(KT_KRYLOV, &ms);

@@ -337,6 +337,7 @@ struct LaunchCfg {
     int olf_allow_resident;
     int smem_3d;          // dynamic shared memory bytes of the 3D solve
     int smem_pipe;        // dynamic shared memory a block of the pipelined solve may take
+    int krylov_solver;    // asked for: 0 by choose_solver's rule, 1 the pipeline, 2 krylov_solve
     int pipe;             // 1: the solves run as the pipeline (pipe_solve.cuh)
     int nz_max;
     int mixed;
@@ -428,4 +429,5 @@ cudaError_t launch_layer_stats(const DevPtrs &P, double *part, int nz_max, doubl
                                cudaStream_t s);
 
 cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom);
+void choose_solver(LaunchCfg &L, int ntiles, int ndom);
 cudaError_t configure_2d(LaunchCfg &L, int device);

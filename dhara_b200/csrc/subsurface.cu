@@ -1663,7 +1663,7 @@ const void *pipe_kernel(const LaunchCfg &L, bool step) {
 // fewer.  Two column buffers when blocks have more than one tile and a ring of
 // PIPE_RING_LEAST stages still fits beside them (fewer keep too few bytes in
 // flight); the ring takes the rest, up to a whole column where a block has one
-// tile.  False where no such ring fits (columns of over 48 layers in FP64 mode).
+// tile.  False where no such ring fits (columns of over 50 layers in FP64 mode).
 #define PIPE_RING_LEAST 6
 // shared memory the kernels declare: PipeShared and the step phases' reductions
 #define PIPE_STATIC_SMEM ((int)sizeof(pipe::PipeShared) + 2048)
@@ -1712,6 +1712,16 @@ bool use_pipe(const LaunchCfg &L, int ntiles, int ndom) {
     const int rounds = (ntiles + L.coop_blocks_3d - 1) / L.coop_blocks_3d;
     const double round = L.mixed ? 6.4 : ndom > 1 ? 3.3 : 3.7;
     return tiles <= 26 && tiles <= round * rounds && pipe_shapes(L, ntiles, c, r, smem);
+}
+
+// The solver of a handle's tiles; a pipeline asked for that does not fit runs as
+// krylov_solve.
+void choose_solver(LaunchCfg &L, int ntiles, int ndom) {
+    PipeShape c, r;
+    int smem;
+    L.pipe = L.krylov_solver == 1   ? pipe_shapes(L, ntiles, c, r, smem)
+             : L.krylov_solver == 2 ? 0
+                                    : use_pipe(L, ntiles, ndom);
 }
 
 cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int maxiter, int dirichlet, bool step, cudaStream_t s) {
@@ -1785,7 +1795,7 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom) {
     // 512x512x40 FP64 92 / 84.7), nor for several domains, whose uneven tiles the fused
     // kernel's blocks share less well (256 domains 250 / 235; one domain of
     // 1024x1024x50 320 / 327, of 512x512x40 59.1 / 58.8)
-    L.pipe = use_pipe(L, ntiles, ndom);
+    choose_solver(L, ntiles, ndom);
     L.fused_step = !L.pipe && ndom == 1 && L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
     return cudaSuccess;
 }

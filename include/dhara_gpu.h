@@ -308,8 +308,9 @@ int dhara_get_krylov_traffic(dhara_handle *h, double *bytes, int64_t *iterations
  * rounding (reductions run over tiles in a fixed order; a different tile
  * shape groups the sums differently), and bit for bit across block counts.
  * Handles with few tiles per SM run the Krylov solve as a pipeline of one block
- * per SM whatever the block count; a domain's results in such a handle and in a
- * larger one agree to rounding. */
+ * per SM whatever the block count (krylov_solver); a domain's results in such a
+ * handle and in a larger one agree to rounding, and bit for bit where both have
+ * the same solver. */
 typedef struct {
     int32_t krylov_blocks_per_sm;
     int32_t overland_resident;
@@ -327,7 +328,11 @@ typedef struct {
      * per kernel (per-kernel timing then names every phase).  Results are the
      * same bit for bit. */
     int32_t fused_step;
-    int32_t pad;
+    /* the Krylov solve: 1 = the pipeline, 2 = krylov_blocks_per_sm blocks per SM.
+     * Read: the one that runs.  Set: 1 or 2 asks for it (2 runs where the columns are
+     * too tall for the pipeline's shared memory), any other value chooses by the
+     * tiles per SM -- the default, decided again when tile_shape changes. */
+    int32_t krylov_solver;
 } dhara_launch_config;
 
 int dhara_autotune(dhara_handle *h, int trial_steps, dhara_launch_config *chosen);
