@@ -214,12 +214,13 @@ void collect_timing(dhara_handle *h) {
 
 // With a tape (the adjoint's recompute sweep), every Picard iterate psi^m and
 // solution x^m is copied into the tape slot after its solve, so the step runs
-// as separate launches; otherwise, with the fused schedule, as one k_step.
+// as separate launches; otherwise, with the fused schedule, as one k_step, and
+// without it the iterations of a small handle that are hardly ever needed.
 int enqueue_subsurface(dhara_handle *h, const AdjPtrs *tape = nullptr, int slot = 0) {
     const DevPtrs &P = h->P;
     cudaStream_t s = h->stream;
     if (!tape && h->L.fused_step) {
-        LAUNCH(KT_STEP, launch_step(P, h->L, h->maxiter_picard, h->any_dirichlet ? 1 : 0, s));
+        LAUNCH(KT_STEP, launch_step(P, h->L, 0, h->maxiter_picard, h->any_dirichlet ? 1 : 0, s));
         if (h->stats_steps > 0) {
             LAUNCH(KT_EPILOGUE, launch_layer_stats(P, h->stats_part, h->nz_max, h->stats_hist, h->stats_steps, s));
             h->launch_count += 1;  // the statistics are two kernels
@@ -227,7 +228,8 @@ int enqueue_subsurface(dhara_handle *h, const AdjPtrs *tape = nullptr, int slot 
         return DHARA_OK;
     }
     LAUNCH(KT_PROLOGUE, launch_prologue(P, s));
-    for (int m = 0; m < h->maxiter_picard; ++m) {
+    const int own = tape ? h->maxiter_picard : separate_iterations(h->L, P.ntiles, h->maxiter_picard);
+    for (int m = 0; m < own; ++m) {
         LAUNCH(KT_ASSEMBLE, launch_assemble(P, h->L, s));
         if (h->any_dirichlet) {
             LAUNCH(KT_ASSEMBLE, launch_dirichlet(P, h->L, s));
@@ -241,6 +243,8 @@ int enqueue_subsurface(dhara_handle *h, const AdjPtrs *tape = nullptr, int slot 
         }
         LAUNCH(KT_CHECK, launch_picard_check(P, s));
     }
+    if (own < h->maxiter_picard)
+        LAUNCH(KT_STEP, launch_step(P, h->L, own, h->maxiter_picard, h->any_dirichlet ? 1 : 0, s));
     LAUNCH(KT_EPILOGUE, launch_epilogue(P, h->L, s));
     if (h->stats_steps > 0) {
         LAUNCH(KT_EPILOGUE, launch_layer_stats(P, h->stats_part, h->nz_max, h->stats_hist, h->stats_steps, s));

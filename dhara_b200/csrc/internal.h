@@ -355,7 +355,10 @@ cudaError_t launch_assemble(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s
 cudaError_t launch_krylov(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s);
 // prologue, Picard loop (assembly, Dirichlet passes, solve, check) and
 // epilogue of a subsurface step in one persistent launch
-cudaError_t launch_step(const DevPtrs &P, const LaunchCfg &L, int maxiter, int dirichlet, cudaStream_t s);
+// The Picard iterations from `first` on in one launch; with the prologue and the
+// epilogue (a whole step) when that is 0.
+cudaError_t launch_step(const DevPtrs &P, const LaunchCfg &L, int first, int maxiter, int dirichlet, cudaStream_t s);
+int separate_iterations(const LaunchCfg &L, int ntiles, int maxiter);
 cudaError_t launch_dirichlet(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s);
 cudaError_t launch_picard_check(const DevPtrs &P, cudaStream_t s);
 cudaError_t launch_epilogue(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s);

@@ -1448,12 +1448,18 @@ __device__ __noinline__ void step_phase(const DevPtrs &P) {
     }
 }
 
-// solve(): the linear solve of one Picard iteration.
+// solve(): the linear solve of one Picard iteration.  first: 0 for a whole step, else
+// the Picard iterations from `first` on, if any domain needs them, without the
+// prologue and the epilogue.
 template <typename T, int GROUPS, typename Solve>
-__device__ __forceinline__ void run_step(const DevPtrs &P, int maxiter, int dirichlet, Solve solve) {
-    step_phase<T, PH_PROLOGUE, GROUPS>(P);
-    if (!grid_sync(P.barrier)) return;
-    for (int m = 0; m < maxiter; ++m) {
+__device__ __forceinline__ void run_step(const DevPtrs &P, int first, int maxiter, int dirichlet, Solve solve) {
+    if (first == 0) {
+        step_phase<T, PH_PROLOGUE, GROUPS>(P);
+        if (!grid_sync(P.barrier)) return;
+    } else if (ldcg(&P.gctrl->n_picard) == 0) {
+        return;
+    }
+    for (int m = first; m < maxiter; ++m) {
         step_phase<T, PH_ASSEMBLE, GROUPS>(P);
         if (!grid_sync(P.barrier)) return;
         if (dirichlet) {
@@ -1467,18 +1473,18 @@ __device__ __forceinline__ void run_step(const DevPtrs &P, int maxiter, int diri
         if (!grid_sync(P.barrier)) return;
         if (ldcg(&P.gctrl->n_picard) == 0) break;
     }
-    step_phase<T, PH_EPILOGUE, GROUPS>(P);
+    if (first == 0) step_phase<T, PH_EPILOGUE, GROUPS>(P);
 }
 
 template <typename T, int TXC>
 __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? KRYLOV_BLOCKS_F32 : KRYLOV_BLOCKS_F64)
-    k_step(const __grid_constant__ DevPtrs P, int maxiter, int dirichlet) {
+    k_step(const __grid_constant__ DevPtrs P, int first, int maxiter, int dirichlet) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t s_bar[STAGES];
     constexpr bool DSMEM = sizeof(T) == 4 && KRYLOV_DSMEM_F32;
     const SolveSmem<T> sm = solve_smem<T, DSMEM>(P, smem_raw, s_bar);
     StageBars sb{s_bar, 0u, P.barrier, 0u};
-    run_step<T, 1>(P, maxiter, dirichlet, [&]() { return krylov_solve<T, DSMEM, TXC>(P, sm, sb); });
+    run_step<T, 1>(P, first, maxiter, dirichlet, [&]() { return krylov_solve<T, DSMEM, TXC>(P, sm, sb); });
 }
 
 // The same kernels with the pipelined solve.
@@ -1491,11 +1497,11 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_krylov_pipe(const __grid_c
 }
 template <typename T, int TXC>
 __global__ void __launch_bounds__(SOLVE_THREADS, 1)
-    k_step_pipe(const __grid_constant__ DevPtrs P, int maxiter, int dirichlet) {
+    k_step_pipe(const __grid_constant__ DevPtrs P, int first, int maxiter, int dirichlet) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) pipe::PipeShared sh;
     pipe::SolveBlock b = pipe::solve_block(P, smem_raw, &sh);
-    run_step<T, STEP_GROUPS>(P, maxiter, dirichlet, [&]() { return pipe::solve<T, TXC>(P, b); });
+    run_step<T, STEP_GROUPS>(P, first, maxiter, dirichlet, [&]() { return pipe::solve<T, TXC>(P, b); });
 }
 
 // Evaluates the closure at psi^n into out: which = 0 theta, 1 K, 2 C.
@@ -1659,6 +1665,18 @@ const void *pipe_kernel(const LaunchCfg &L, bool step) {
                                   : pipe_fn<0>(L.mixed, step);
 }
 
+// Picard iterations of a step that get launches of their own in the launch-per-kernel
+// schedule; the rest share one, which ends its loop on the device.  An iteration is
+// queued whether or not it is needed, and three launches that find nothing to do take
+// 8 us from a graph and 14 us without one: 32x32x20 FP64 with two iterations of up to
+// 100 took 1.68 and 2.36 ms a step (krylov_solve in the fused step 1.30).  An iteration
+// in the shared launch is slower than one in its own (that domain 0.22 / 0.09 ms,
+// 128x128x30 0.24 / 0.16), so it comes after as many as a step is likely to need, and
+// not in larger handles, where idle launches are little beside an iteration.
+int separate_iterations(const LaunchCfg &L, int ntiles, int maxiter) {
+    return ntiles <= 4 * L.sms && maxiter > 32 ? 32 : maxiter;
+}
+
 // Pipelines and grid of a solve: one block per SM, or per tile where there are
 // fewer.  Two column buffers when blocks have more than one tile and a ring of
 // PIPE_RING_LEAST stages still fits beside them (fewer keep too few bytes in
@@ -1724,7 +1742,8 @@ void choose_solver(LaunchCfg &L, int ntiles, int ndom) {
                                     : use_pipe(L, ntiles, ndom);
 }
 
-cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int maxiter, int dirichlet, bool step, cudaStream_t s) {
+cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int first, int maxiter, int dirichlet, bool step,
+                        cudaStream_t s) {
     DevPtrs args = P;
     int smem = 0;
     const int grid = L.sms < P.ntiles ? L.sms : P.ntiles;
@@ -1732,12 +1751,12 @@ cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int maxiter, int d
     const void *fn = pipe_kernel(L, step);
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem_pipe);
     if (e != cudaSuccess) return e;
-    void *kargs[] = {&args, &maxiter, &dirichlet};
+    void *kargs[] = {&args, &first, &maxiter, &dirichlet};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SOLVE_THREADS), kargs, (size_t)smem, s);
 }
 
 cudaError_t launch_krylov(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s) {
-    if (L.pipe) return launch_pipe(P, L, 0, 0, false, s);
+    if (L.pipe) return launch_pipe(P, L, 0, 0, 0, false, s);
     DevPtrs args = P;
     void *kargs[] = {&args};
     const int blocks = L.krylov_per_sm * L.sms;
@@ -1746,10 +1765,10 @@ cudaError_t launch_krylov(const DevPtrs &P, const LaunchCfg &L, cudaStream_t s) 
                                        (size_t)L.smem_3d, s);
 }
 
-cudaError_t launch_step(const DevPtrs &P, const LaunchCfg &L, int maxiter, int dirichlet, cudaStream_t s) {
-    if (L.pipe) return launch_pipe(P, L, maxiter, dirichlet, true, s);
+cudaError_t launch_step(const DevPtrs &P, const LaunchCfg &L, int first, int maxiter, int dirichlet, cudaStream_t s) {
+    if (L.pipe) return launch_pipe(P, L, first, maxiter, dirichlet, true, s);
     DevPtrs args = P;
-    void *kargs[] = {&args, &maxiter, &dirichlet};
+    void *kargs[] = {&args, &first, &maxiter, &dirichlet};
     const int blocks = (L.krylov_per_sm < L.step_per_sm ? L.krylov_per_sm : L.step_per_sm) * L.sms;
     const int grid = blocks < P.ntiles ? blocks : P.ntiles;
     return cudaLaunchCooperativeKernel(step_kernel(L, L.uniform_tx), dim3(grid), dim3(TILE_THREADS), kargs,

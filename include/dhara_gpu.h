@@ -325,7 +325,8 @@ typedef struct {
      * iteration's assembly, solve and check, epilogue) -- the default where
      * that kernel runs as many blocks per SM as the Krylov kernel and the handle
      * has one domain and not the pipelined solve; 0: a launch
-     * per kernel (per-kernel timing then names every phase).  Results are the
+     * per kernel (per-kernel timing then names every phase; in small handles the
+     * Picard iterations after the 32nd share one launch, counted as a step).  Results are the
      * same bit for bit. */
     int32_t fused_step;
     /* the Krylov solve: 1 = the pipeline, 2 = krylov_blocks_per_sm blocks per SM.
