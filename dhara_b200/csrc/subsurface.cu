@@ -1495,13 +1495,13 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_krylov_pipe(const __grid_c
     pipe::SolveBlock b = pipe::solve_block(P, smem_raw, &sh);
     pipe::solve<T, TXC>(P, b);
 }
-template <typename T, int TXC>
+template <typename T>
 __global__ void __launch_bounds__(SOLVE_THREADS, 1)
     k_step_pipe(const __grid_constant__ DevPtrs P, int first, int maxiter, int dirichlet) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) pipe::PipeShared sh;
     pipe::SolveBlock b = pipe::solve_block(P, smem_raw, &sh);
-    run_step<T, STEP_GROUPS>(P, first, maxiter, dirichlet, [&]() { return pipe::solve<T, TXC>(P, b); });
+    run_step<T, STEP_GROUPS>(P, first, maxiter, dirichlet, [&]() { return pipe::solve<T, 0>(P, b); });
 }
 
 // Evaluates the closure at psi^n into out: which = 0 theta, 1 K, 2 C.
@@ -1655,14 +1655,14 @@ const void *step_kernel(const LaunchCfg &L, int uniform_tx) {
 }
 
 template <int TXC>
-const void *pipe_fn(int mixed, bool step) {
-    return step ? (mixed ? (const void *)k_step_pipe<float, TXC> : (const void *)k_step_pipe<double, TXC>)
-                : (mixed ? (const void *)k_krylov_pipe<float, TXC> : (const void *)k_krylov_pipe<double, TXC>);
+const void *pipe_fn(int mixed) {
+    return mixed ? (const void *)k_krylov_pipe<float, TXC> : (const void *)k_krylov_pipe<double, TXC>;
 }
 const void *pipe_kernel(const LaunchCfg &L, bool step) {
-    return L.uniform_tx == TILE_X ? pipe_fn<TILE_X>(L.mixed, step)
-           : L.uniform_tx == 16   ? pipe_fn<16>(L.mixed, step)
-                                  : pipe_fn<0>(L.mixed, step);
+    if (step) return L.mixed ? (const void *)k_step_pipe<float> : (const void *)k_step_pipe<double>;
+    return L.uniform_tx == TILE_X ? pipe_fn<TILE_X>(L.mixed)
+           : L.uniform_tx == 16   ? pipe_fn<16>(L.mixed)
+                                  : pipe_fn<0>(L.mixed);
 }
 
 // Picard iterations of a step that get launches of their own in the launch-per-kernel
