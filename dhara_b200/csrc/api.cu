@@ -378,7 +378,7 @@ int apply_tiles(dhara_handle *h) {
     CK(cudaMemcpyAsync((void *)h->P.tiles, h->htiles.data(), sizeof(TileDesc) * h->htiles.size(),
                        cudaMemcpyHostToDevice, h->stream));
     h->P.ntiles = (int)h->htiles.size();
-    choose_solver(h->L, h->P.ntiles, h->ndom);
+    CK(choose_solver(h->L, h->P.ntiles, h->ndom));
     int rc = upload_dom_desc(h);
     if (!rc) rc = build_tensor_maps(h);
     if (h->graph_exec) {
@@ -1851,7 +1851,7 @@ int dhara_set_launch_config(dhara_handle *h, const dhara_launch_config *cfg) {
         if (rc) return rc;
     }
     h->L.krylov_solver = cfg->krylov_solver == 1 || cfg->krylov_solver == 2 ? cfg->krylov_solver : 0;
-    choose_solver(h->L, h->P.ntiles, h->ndom);
+    CK(choose_solver(h->L, h->P.ntiles, h->ndom));
     h->L.krylov_per_sm = cfg->krylov_blocks_per_sm;
     h->L.fused_step = cfg->fused_step ? 1 : 0;
     h->L.olf_allow_resident = cfg->overland_resident ? 1 : 0;

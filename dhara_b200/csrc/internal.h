@@ -432,5 +432,5 @@ cudaError_t launch_layer_stats(const DevPtrs &P, double *part, int nz_max, doubl
                                cudaStream_t s);
 
 cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom);
-void choose_solver(LaunchCfg &L, int ntiles, int ndom);
+cudaError_t choose_solver(LaunchCfg &L, int ntiles, int ndom);
 cudaError_t configure_2d(LaunchCfg &L, int device);

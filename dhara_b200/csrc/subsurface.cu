@@ -1733,13 +1733,16 @@ bool use_pipe(const LaunchCfg &L, int ntiles, int ndom) {
 }
 
 // The solver of a handle's tiles; a pipeline asked for that does not fit runs as
-// krylov_solve.
-void choose_solver(LaunchCfg &L, int ntiles, int ndom) {
+// krylov_solve.  The pipeline's kernel is loaded here, so that the first step, or the
+// first capture, does not wait for it (0.1 ms).
+cudaError_t choose_solver(LaunchCfg &L, int ntiles, int ndom) {
     PipeShape c, r;
     int smem;
     L.pipe = L.krylov_solver == 1   ? pipe_shapes(L, ntiles, c, r, smem)
              : L.krylov_solver == 2 ? 0
                                     : use_pipe(L, ntiles, ndom);
+    if (!L.pipe) return cudaSuccess;
+    return cudaFuncSetAttribute(pipe_kernel(L, false), cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem_pipe);
 }
 
 cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int first, int maxiter, int dirichlet, bool step,
@@ -1749,8 +1752,10 @@ cudaError_t launch_pipe(const DevPtrs &P, const LaunchCfg &L, int first, int max
     const int grid = L.sms < P.ntiles ? L.sms : P.ntiles;
     if (!pipe_shapes(L, P.ntiles, args.pipe_c, args.pipe_r, smem)) return cudaErrorInvalidConfiguration;
     const void *fn = pipe_kernel(L, step);
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem_pipe);
-    if (e != cudaSuccess) return e;
+    if (step) {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem_pipe);
+        if (e != cudaSuccess) return e;
+    }
     void *kargs[] = {&args, &first, &maxiter, &dirichlet};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SOLVE_THREADS), kargs, (size_t)smem, s);
 }
@@ -1799,8 +1804,6 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom) {
         }
     }
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    // the pipeline's kernels are not set up here: each is loaded when it is first
-    // launched (all six cost 19 ms of a process's first handle)
     L.smem_pipe = (int)prop.sharedMemPerBlockOptin - PIPE_STATIC_SMEM;
     L.coop_blocks_3d = per_sm * prop.multiProcessorCount;
     L.sms = prop.multiProcessorCount;
@@ -1814,7 +1817,7 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom) {
     // 512x512x40 FP64 92 / 84.7), nor for several domains, whose uneven tiles the fused
     // kernel's blocks share less well (256 domains 250 / 235; one domain of
     // 1024x1024x50 320 / 327, of 512x512x40 59.1 / 58.8)
-    choose_solver(L, ntiles, ndom);
+    e = choose_solver(L, ntiles, ndom);
     L.fused_step = !L.pipe && ndom == 1 && L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
-    return cudaSuccess;
+    return e;
 }
