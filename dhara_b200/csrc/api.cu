@@ -691,7 +691,7 @@ int dhara_create(const dhara_params *params, int ndomains, int device, dhara_han
         D.picard_maxiter = p.picard_maxiter; D.krylov_maxiter = p.krylov_maxiter;
         D.overland_maxiter = p.overland_maxiter;
         D.inner_maxiter = h->mixed ? (p.inner_maxiter > 0 ? p.inner_maxiter : p.krylov_maxiter) : p.krylov_maxiter;
-        D.nxp = (p.nx + 7) & ~7;  // rows of every array 16-byte aligned, 2-byte factors included
+        D.nxp = (p.nx + 7) & ~7;  // rows of every array 32-byte aligned
         h->Ntot = (h->Ntot + 31) & ~31LL;  // 128-byte aligned base for FP32 and FP64
         D.off3 = h->Ntot; D.off2 = h->Ctot; D.offWE = h->WEtot; D.offSN = h->SNtot;
         h->Ntot += (long long)D.nxp * p.ny * p.nz;

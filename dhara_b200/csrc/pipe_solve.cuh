@@ -24,8 +24,6 @@
 
 namespace pipe {
 
-static_assert(!FACTOR_NARROW_F32, "the own arrays of a set are of one type in mixed mode");
-
 // columns a 16-byte unit of an array holds: the x offset of a halo box
 template <typename V>
 __host__ __device__ constexpr int xoff() {

@@ -22,8 +22,8 @@
 
 #include <cstdio>
 
-// Storage type of the column preconditioner's factors 1/den and c': bf16 in
-// mixed mode with FACTOR_NARROW_F32, FP32 in FP64 mode with FACTOR_NARROW_F64.  Any rounding of
+// Storage type of the column preconditioner's factors 1/den and c': FP32 in FP64
+// mode too with FACTOR_NARROW_F64.  Any rounding of
 // the stored pair still defines a symmetric positive definite M = L D L^T
 // (D = 1/inv > 0, L from c'), and every use of M -- phase R's z = M^-1 r,
 // the sweep's forward and back substitutions and its z.M z -- goes through
@@ -32,12 +32,6 @@ template <typename T>
 struct Fac {
     using type = T;
 };
-#if FACTOR_NARROW_F32
-template <>
-struct Fac<float> {
-    using type = __nv_bfloat16;
-};
-#endif
 #if FACTOR_NARROW_F64
 template <>
 struct Fac<double> {
@@ -547,17 +541,6 @@ struct Chunk {
     static constexpr int inner = sizeof(T) == 4 ? CHUNK_F32 : CHUNK_F64;
 };
 
-template <typename T, typename F>
-__device__ __forceinline__ T fac_get(F v) {
-    if constexpr (std::is_same<F, __nv_bfloat16>::value) return (T)__bfloat162float(v);
-    else return (T)v;
-}
-template <typename F, typename T>
-__device__ __forceinline__ F fac_put(T v) {
-    if constexpr (std::is_same<F, __nv_bfloat16>::value) return __float2bfloat16_rn((float)v);
-    else return (F)v;
-}
-
 // Bytes of one staging buffer of each phase (the kernel reserves STAGES buffers
 // of the largest).
 template <typename T>
@@ -657,7 +640,7 @@ __device__ __forceinline__ void back_sweep(const ColumnRef &cr, const T *s_d, co
             const int k = k0 - q;
             if (k >= 0) {
                 const unsigned g = g0 + (unsigned)k * sxy;
-                cl[q] = fac_get<T>(fc[g]);
+                cl[q] = (T)fc[g];
                 dl[q] = DSMEM ? s_d[k * TILE_THREADS + threadIdx.x] : z[g];
             }
         }
@@ -862,10 +845,10 @@ __device__ __forceinline__ void phase_R(const DevPtrs &P, int tile, int tile_nex
         const T bd = (lateral_diag((T)Dk, fw, fe, fs, fn) + fd) + fu;
         const T den = bd + fd * cprev;  // b_k - a_k c'_{k-1} with a_k = -fd
         // the stored (rounded) factors are the ones applied, here as in the sweeps
-        const F inv_s = fac_put<F>(fixed ? T(0) : recip(den));
-        const T inv = fac_get<T>(inv_s);
-        const F cp_s = fac_put<F>(-fu * inv);
-        const T cp = fac_get<T>(cp_s);
+        const F inv_s = (F)(fixed ? T(0) : recip(den));
+        const T inv = (T)inv_s;
+        const F cp_s = (F)(-fu * inv);
+        const T cp = (T)cp_s;
         const T y = rT - cprev * yprev;
         const T dp = y * inv;
         finv[g] = inv_s;
@@ -961,7 +944,7 @@ __device__ __forceinline__ void phase_C(const DevPtrs &P, int tile, int tile_nex
                 pc = pz(zc, sp, hc);
                 Kc = sK[hc];
             }
-            const T Dk = ownD[0], inv = fac_get<T>(ownI[0]), cp = fac_get<T>(ownC[0]);
+            const T Dk = ownD[0], inv = (T)ownI[0], cp = (T)ownC[0];
             T z_dn = T(0), p_dn = T(0), K_dn = T(0), fu = T(0);
             if (k + 1 < nz) {
                 const T *nzz = sz + H.plane, *ntt = st + H.plane, *npp = sp + H.plane, *nK = sK + H.plane;
