@@ -130,11 +130,15 @@ struct StageR {
     static constexpr unsigned x = 0, K = hs, D = 2 * hs, b = D + ob, inv = b + ob, c = inv + of, bytes = c + of;
 };
 // A column buffer: of every cell of a tile's columns, plane by plane, the right-
-// hand side of the column solve in T and then, in 8 bytes, the factors c' and
-// 1/den (two arrays of F), or in a solve's first phase R the matrix they are
-// formed from: in FP32 the vertical coupling and the diagonal, in FP64 the
-// diagonal (the coupling is then left in the d array, which is free there).
-__host__ __device__ constexpr int col_bytes(int nz, int elt) { return TILE_THREADS * (elt + 8) * nz; }
+// hand side of the column solve in T and then the factors c' and 1/den (two arrays
+// of F), or in a solve's first phase R the matrix they are formed from: in FP32 the
+// vertical coupling and the diagonal, in FP64 the diagonal (the coupling is then
+// left in the d array, which is free there).
+template <typename T>
+__host__ __device__ constexpr int col_bytes(int nz) {
+    constexpr int factors = 2 * (int)sizeof(typename Fac<T>::type), matrix = (sizeof(T) == 4 ? 2 : 1) * (int)sizeof(T);
+    return TILE_THREADS * ((int)sizeof(T) + (factors > matrix ? factors : matrix)) * nz;
+}
 
 // What the roles need to know of a tile.  A block's first TILE_TABLE tiles are
 // kept in shared memory for the whole solve: each sweep starts with a grid

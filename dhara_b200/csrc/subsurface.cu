@@ -1673,7 +1673,7 @@ bool pipe_shapes(const LaunchCfg &L, int ntiles, PipeShape &c, PipeShape &r, int
     const int room = L.smem_pipe - 128;  // alignment
     c.stage = (int)pipe::Stage<T>::bytes;
     r.stage = (int)pipe::StageR<T>::bytes;
-    c.colb = r.colb = pipe::col_bytes(L.nz_max, sizeof(T));
+    c.colb = r.colb = pipe::col_bytes<T>(L.nz_max);
     const int whole = pipe::units_of(L.nz_max) < 3 ? 3 : pipe::units_of(L.nz_max);
     const int most = ntiles > L.sms ? RING_MAX : whole;
     bool fits = true;
