@@ -41,7 +41,7 @@ def gather_diagnostics(local, world):
     return merged
 
 
-def run_sharded(domains, nsteps, rank, world, device=0, graph=True, autotune=0):
+def run_sharded(domains, nsteps, rank, world, device=0, graph=True, autotune=0, krylov_solver=2):
     """Advances this rank's share of `domains` (inputs.Domain objects) for
     nsteps in one handle on `device`; returns this rank's device time in ms
     (CUDA events on the handle's stream), the number of kernel launches it
@@ -49,7 +49,12 @@ def run_sharded(domains, nsteps, rank, world, device=0, graph=True, autotune=0):
     |psi| after the run, "psi_abs_max", and under "launch_config" the
     schedule used), gathered from every rank.  autotune > 0 first lets
     dhara_autotune choose the tile shapes and schedules with that many trial
-    steps (the state is restored before the timed run)."""
+    steps (the state is restored before the timed run).  krylov_solver is the
+    3D solver of every rank's handle (dhara_launch_config): the same one
+    everywhere, so that a domain's results are the same bits for any number of
+    ranks.  1, the pipeline, is faster in small shares (32 of the benchmark's
+    256 domains 41 ms a step against 63) and slower in large ones; 0 lets each
+    handle choose by its own size, and results agree to rounding only."""
     import torch
     import dhara_b200 as db
     cells = [d.ncells for d in domains]
@@ -62,6 +67,9 @@ def run_sharded(domains, nsteps, rank, world, device=0, graph=True, autotune=0):
             for j, i in enumerate(mine):
                 s.load(domains[i], j)
             s.prepare()
+            c = s.launch_config()
+            s.set_launch_config(c["krylov_blocks_per_sm"], c["overland_resident"], c["overland_blocks_per_sm"],
+                                krylov_solver=krylov_solver)
             cfg = s.autotune(autotune) if autotune > 0 else s.launch_config()
             stream = torch.cuda.ExternalStream(s.stream, device=device)
             e0 = torch.cuda.Event(enable_timing=True)
