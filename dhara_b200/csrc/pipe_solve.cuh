@@ -9,11 +9,12 @@
 // of a tile are computed by different warps at the same time, since only the two
 // recurrences of the column solve have an order in k, and these run from shared
 // memory.  All solves of a pass, krylov_solve / this in ms: 32x32x20 FP64 two steps
-// 3.73 / 2.09, 53x37x21 FP64 2.17 / 1.18, 128x128x30 5.38 / 2.62, 301x211x33 14.9 /
-// 12.7, 384x384x40 48.0 / 32.9, 512x512x40 FP64 78.2 / 71.2.  What bounds it: in
-// small handles the chain of a sweep (issue of the copies, recurrences, sums, grid
-// barrier); in larger ones the instructions of the plane warps, which krylov_solve
-// spreads over 28 warps per SM -- it keeps those handles (use_pipe).
+// 3.77 / 2.24, 53x37x21 FP64 2.16 / 1.22, 128x128x30 5.36 / 2.65, 384x384x40 48.8 /
+// 33.2; more sizes at use_pipe.  What bounds it: in small handles the chain of a sweep
+// (issue of the copies, recurrences, sums, grid barrier; 128x128x30 issues in 27 % of
+// the cycles); in larger ones the chains of the plane warps' instructions, of which an
+// SM has eight (384x384x40: issue 41 %, DRAM 39 % of peak).  krylov_solve spreads them
+// over 28 warps per SM -- it keeps the largest handles (use_pipe).
 #pragma once
 
 #include "device_common.cuh"

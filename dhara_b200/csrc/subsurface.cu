@@ -1698,14 +1698,14 @@ bool pipe_shapes(const LaunchCfg &L, int ntiles, PipeShape &c, PipeShape &r, int
 // its blocks make: measured, a round takes as long as 6.4 tiles of the pipeline
 // (mixed), 3.7 (FP64 mode; 3.3 where a block's tiles are of several domains, whose
 // sums are formed one after the other).  Solves of a pass, krylov_solve / pipeline
-// in ms, tiles per SM (t) against rounds (r): mixed 301x211x33 14.9 / 12.5 (t 5, r
-// 1), 384x384x40 48.0 / 32.9 (8, 2), 448x448x40 50.0 / 45.0 (11, 2), 512x512x40 50.9
-// / 53.5 (14, 2), 576x576x40 80.3 / 78.2 (18, 3), 700x700x40 103 / 113 (27, 4); 64
-// domains 59.8 / 53.6 (19, 3), 80 71.6 / 73.8 (26, 4); FP64 272x272x40 21.9 / 22.9
-// (4, 1), 400x400x40 59.4 / 48.6 (9, 3), 512x512x40 76.0 / 71.2 (14, 4), 640x640x40
-// 127 / 122 (22, 6), 768x768x40 169 / 169 (32, 8); 48 domains 18.3 / 17.2 (6, 2), 64
-// 18.3 / 19.7 (7, 2).  Above 26 tiles per SM the two are within 5 % or krylov_solve
-// is ahead (256 domains 192 / 210).
+// in ms, tiles per SM (t) against rounds (r): mixed 301x211x33 14.7 / 12.8 (t 4, r
+// 1), 384x384x40 48.8 / 33.2 (8, 2), 448x448x40 50.2 / 44.6 (11, 2), 512x512x40 51.7
+// / 53.5 (14, 2), 576x576x40 81.2 / 78.0 (18, 3), 640x640x40 102 / 91.9 (22, 4),
+// 700x700x40 107 / 113 (27, 4); 64 domains 59.3 / 50.5 (19, 3), 80 71.6 / 72.3 (26,
+// 4); FP64 272x272x40 22.0 / 23.0 (4, 1), 400x400x40 59.7 / 49.2 (9, 3), 512x512x40
+// 78.2 / 74.2 (14, 4), 640x640x40 131 / 128 (22, 6), 768x768x40 171 / 172 (32, 8); 48
+// domains of up to 64x64x30 19.2 / 17.0 (6, 2), 64 18.4 / 20.2 (7, 2).  Above 26 tiles
+// per SM the two are within 5 % or krylov_solve is ahead (256 domains 189 / 212).
 bool use_pipe(const LaunchCfg &L, int ntiles, int ndom) {
     PipeShape c, r;
     int smem;
@@ -1795,11 +1795,11 @@ cudaError_t configure_3d(LaunchCfg &L, int device, int ntiles, int ndom) {
     L.step_per_sm = step_sm < per_sm ? step_sm : per_sm;
     if (L.step_per_sm < 1) return cudaErrorInvalidConfiguration;
     // one launch per subsurface step by default, where the fused kernel keeps the
-    // Krylov kernel's occupancy, but not with the pipelined solve, whose block has too
-    // few warps for the assembly (32x32x20 FP64 two steps 6.1 fused, 5.75 ms separate,
-    // 512x512x40 FP64 92 / 84.7), nor for several domains, whose uneven tiles the fused
-    // kernel's blocks share less well (256 domains 250 / 235; one domain of
-    // 1024x1024x50 320 / 327, of 512x512x40 59.1 / 58.8)
+    // Krylov kernel's occupancy, but not with the pipelined solve, whose grid has too
+    // few warps for the assembly (a step of 32x32x20 FP64 2.58 ms fused, 1.32 separate,
+    // 128x128x30 4.52 / 3.69, 512x512x40 FP64 64.5 / 57.7), nor for several domains,
+    // whose uneven tiles the fused kernel's blocks share less well (256 domains 237 /
+    // 222; one domain of 1024x1024x50 320 / 327, of 512x512x40 59.1 / 58.8)
     e = choose_solver(L, ntiles, ndom);
     L.fused_step = !L.pipe && ndom == 1 && L.step_per_sm >= L.krylov_per_sm ? 1 : 0;
     return e;
